@@ -18,7 +18,8 @@ with them from the autotuner's cache); empty: the library's own defaults.
 Solvent: about ``n_c`` particles per cell, uniform, Maxwell-Boltzmann at kT = 1; stars: self-avoiding walks in a random
 orientation, mass 5 beads, half of them solvophobic. The 12-6 preset with skin 0.3 and 10 substeps of 0.01 per
 collision (h = 0.1), as the workloads of ``starpolymersmd_gb300.workloads``; ``dropin`` runs the reference's own 48-24
-potentials and options.
+potentials and options. What an FP32 context gives (its observables too, whose sums are in 64 bits) is compared as the
+float32 numbers that its state holds.
 """
 from __future__ import annotations
 
@@ -100,7 +101,8 @@ def draw(rng):
     if what == "amc":
         return _case("cycles", "star", L=_log(rng, 17, 50), arms=arms, n_arm=min(n_arm, 30), shear=shear, fp64=fp64, amc=True)
     if what == "md":
-        return _case("md", "star", L=50, arms=arms, n_arm=n_arm, fp64=rng.random() < 0.5, steps=_log(rng, 20, 200))
+        fp64 = rng.random() < 0.5  # FP32 trajectories part from each other after some tens of substeps
+        return _case("md", "star", L=50, arms=arms, n_arm=n_arm, fp64=fp64, steps=_log(rng, 20, 200) if fp64 else _log(rng, 10, 30))
     if what == "dropin":
         return _case("dropin", "star", L=_log(rng, 20, 40), arms=rng.randint(3, 8), n_arm=rng.randint(5, 12), shear=0.01,
                      fp64=True)
@@ -271,7 +273,7 @@ def run(state):
         return {"state": _held(s), "error_word": ctx.error_word()[0]}
     if kind == "io":
         ctx.cycles_io(steps, s["pos"], s["vel"], s["pos"], s["vel"], s["obs"])
-        return {"state": _held(s), "observables": s["obs"]}
+        return {"state": _held(s), "observables": s["obs"].astype(s["real"])}
     if kind == "dropin":
         for _ in range(N_SUB):
             ctx.md_substeps(1)
@@ -280,7 +282,7 @@ def run(state):
         return _held(s)
     if kind == "md":
         ctx.md_substeps(steps, calc_epot=True)
-        return {"state": _held(s), "epot": np.array([ctx.epot()])}
+        return {"state": _held(s), "epot": np.array([ctx.epot()], dtype=s["real"])}
     kin, vir = ctx.pressure_tensor_all()
     return {"molecules": ctx.molecule_observables_all(), "profile": ctx.velocity_profile(0, 1.0), "kinetic": kin,
             "virial": vir}
