@@ -4,7 +4,9 @@
 #include <algorithm>
 #include "launch.h"
 #include "md_kernels.cuh"
+#if SMPC_FAST_F32
 #include "mpc_fast.cuh"
+#endif
 #include "mpc_kernels.cuh"
 #include "observables.cuh"
 #include "pmd_kernels.cuh"
@@ -64,33 +66,6 @@ void bin_f32(const Tile* tiles, int n_tiles, const RepInfo* reps, const FrameF* 
                                                           err);
 }
 
-template <int NT, int CT, int CAP, int GU>
-void collide_f32(const CollideArgs<float>& a, cudaStream_t st) {
-  auto kern = k_collide_f32<NT, CT, CAP, GU>;
-  const size_t dyn = collide_f32_dyn_smem(CAP);
-  static bool configured = false;  // the attribute is per function, set once
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
-    configured = true;
-  }
-  kern<<<a.n_tiles, NT, dyn, st>>>(a.tiles, a.reps, a.frames, a.dyn, a.off, a.perm, a.st_in,
-                                   a.st_out, a.mpos, a.mvel, a.mimg, a.inj_gamma, a.inj_uphi,
-                                   a.inj_utheta, a.rng, a.mono_bin, a.err);
-}
-
-template <int NT, int CT, int CAP>
-void collide_f32_async(const CollideArgs<float>& a, cudaStream_t st) {
-  auto kern = k_collide_f32_async<NT, CT, CAP>;
-  const size_t dyn = collide_f32_dyn_smem(CAP);
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
-    configured = true;
-  }
-  kern<<<a.n_tiles, NT, dyn, st>>>(a.tiles, a.reps, a.frames, a.dyn, a.off, a.perm, a.st_in,
-                                   a.st_out, a.mpos, a.mvel, a.mimg, a.inj_gamma, a.inj_uphi,
-                                   a.inj_utheta, a.rng, a.mono_bin, a.err);
-}
 #endif
 
 template <>
@@ -123,20 +98,10 @@ void launch_collide<Real>(const CollideArgs<Real>& a, cudaStream_t st) {
   if (a.n_tiles == 0) return;
 #if SMPC_FAST_F32
   if (!a.strict && !a.amc) {
-    switch (a.variant) {
-      case 1: collide_f32<256, 128, 1408, 8>(a, st); return;
-      case 2: collide_f32<128, 64, 704, 4>(a, st); return;
-      case 3: collide_f32<128, 64, 704, 8>(a, st); return;
-      case 4: collide_f32<512, 256, 2816, 4>(a, st); return;
-      case 5: collide_f32_async<128, 64, 704>(a, st); return;
-      case 6: collide_f32_async<256, 128, 1408>(a, st); return;
-      case 7: collide_f32_async<128, 64, 736>(a, st); return;
-      case 8: collide_f32_async<128, 64, 768>(a, st); return;
-      case 9: collide_f32_async<160, 64, 704>(a, st); return;
-      case 10: collide_f32_async<192, 64, 704>(a, st); return;
-      case 11: collide_f32_async<256, 64, 704>(a, st); return;
-      default: collide_f32<256, 128, 1408, 4>(a, st); return;
-    }
+    k_collide_tile<<<a.n_tiles, COL_NT, 0, st>>>(
+        a.tiles, a.reps, a.frames, a.dyn, a.off, a.perm, a.st_in, a.st_out, a.mpos, a.mvel, a.mimg,
+        a.inj_gamma, a.inj_uphi, a.inj_utheta, a.rng, a.mono_bin, a.err);
+    return;
   }
 #endif
   auto kern = k_collide<Real, SMPC_COLLIDE_NT, SMPC_COLLIDE_CT, SMPC_COLLIDE_CAP>;

@@ -17,7 +17,8 @@ struct PmdArgs;
 int bin_variant_count();
 int collide_variant_count();
 int md_variant_count();
-int collide_variant_cells(int v);     // cells per collide tile of variant v
+int collide_shape_count();            // distinct collide shapes among the variants
+int collide_tile_cells(double density, long long total_cells);  // cells per collide tile
 const char* bin_variant_name(int v);
 const char* collide_variant_name(int v);
 const char* md_variant_name(int v);
@@ -30,7 +31,6 @@ const char* pmd_variant_name(int v);
 
 template <typename R>
 struct CollideArgs {
-  int variant;
   const FrameF* frames;  // float frames (FP32 path)
   const Tile* tiles;
   int n_tiles;

@@ -41,11 +41,8 @@ struct smpc_ctx {
   Tile* d_bin_tiles = nullptr;
   int n_bin_tiles = 0;
   std::vector<int> bin_tile_rep;  // replica of each binning tile
-  Tile* d_col_tiles = nullptr;   // parity-path collide tiles
+  Tile* d_col_tiles = nullptr;   // collide tiles
   int n_col_tiles = 0;
-  // fast path: collide tiles for each tile size the variants use (64/128/256 cells)
-  Tile* d_col_tiles_v[3] = {nullptr, nullptr, nullptr};
-  int n_col_tiles_v[3] = {0, 0, 0};
   int var_bin = 0, var_col = 0, var_md = 0, var_pmd = 0;
   // FP32 fast path, every box at most 65,536 cells: 32-bit sort keys
   bool packed_keys = false;
@@ -156,7 +153,6 @@ namespace {
 bool fast_path(const smpc_ctx* ctx) {
   return ctx->opt.precision == SMPC_FP32 && !ctx->opt.strict_cells && !ctx->opt.angular_momentum;
 }
-int tile_set(int cells) { return cells == 64 ? 0 : (cells == 128 ? 1 : 2); }
 
 int fail(smpc_ctx* c, int code, const std::string& msg) {
   if (c) c->err = msg;
@@ -252,15 +248,9 @@ template <typename R>
 smpc::CollideArgs<R> collide_args(smpc_ctx* ctx, int rng, int cur) {
   const int strict = ctx->opt.strict_cells;
   smpc::CollideArgs<R> a;
-  a.variant = ctx->var_col;
   a.frames = ctx->d_frames;
   a.tiles = ctx->d_col_tiles;
   a.n_tiles = ctx->n_col_tiles;
-  if (fast_path(ctx)) {
-    const int k = tile_set(smpc::collide_variant_cells(ctx->var_col));
-    a.tiles = ctx->d_col_tiles_v[k];
-    a.n_tiles = ctx->n_col_tiles_v[k];
-  }
   a.reps = ctx->d_reps;
   a.dyn = ctx->d_dyn;
   a.off = ctx->d_off;
@@ -771,8 +761,6 @@ void free_all(smpc_ctx* ctx) {
                   ctx->d_mol_rep, ctx->d_init_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  for (int k = 0; k < 3; ++k)
-    if (ctx->d_col_tiles_v[k]) cudaFree(ctx->d_col_tiles_v[k]);
   if (ctx->dyn_ev) cudaEventDestroy(ctx->dyn_ev);
   if (ctx->h_dyn_pinned) cudaFreeHost(ctx->h_dyn_pinned);
   if (ctx->md_split.fork) cudaEventDestroy(ctx->md_split.fork);
@@ -1118,7 +1106,17 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
                                              : smpc::collide_cells_per_tile<float>();
   std::vector<Tile> bin =
       make_tiles(ctx->reps, false, smpc::fluid_slots_per_tile(opt->precision == SMPC_FP64));
-  std::vector<Tile> col = make_tiles(ctx->reps, true, ct);
+  std::vector<Tile> col;
+  if (fast_path(ctx)) {
+    for (const RepInfo& ri : ctx->reps) {
+      const int n = smpc::collide_tile_cells(static_cast<double>(ri.slot_cap) / ri.n_cell, cells);
+      for (int b = 0; b < ri.n_cell; b += n)
+        col.push_back(Tile{static_cast<int>(&ri - ctx->reps.data()), ri.cell_base + b,
+                           ri.cell_base + std::min(ri.n_cell, b + n), 0});
+    }
+  } else {
+    col = make_tiles(ctx->reps, true, ct);
+  }
   ctx->h_tmp_tiles = make_tiles(ctx->reps, true, smpc::temperature_cells_per_tile());
   ctx->n_bin_tiles = static_cast<int>(bin.size());
   for (const Tile& t : bin) ctx->bin_tile_rep.push_back(t.rep);
@@ -1140,17 +1138,6 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
   ctx->packed_keys = fast_path(ctx);
   for (const RepInfo& ri : ctx->reps)
     if (ri.n_cell > 65536) ctx->packed_keys = false;
-  if (fast_path(ctx)) {
-    const int cells[3] = {64, 128, 256};
-    for (int k = 0; k < 3; ++k) {
-      std::vector<Tile> tv = make_tiles(ctx->reps, true, cells[k]);
-      ctx->n_col_tiles_v[k] = static_cast<int>(tv.size());
-      if (dalloc(&ctx->d_col_tiles_v[k], tv.size()) != cudaSuccess ||
-          cudaMemcpy(ctx->d_col_tiles_v[k], tv.data(), tv.size() * sizeof(Tile),
-                     cudaMemcpyHostToDevice) != cudaSuccess)
-        return bail(SMPC_E_CUDA, "tile tables");
-    }
-  }
   // molecules: molecule 0 = the first mol0_size monomers (the recentring
   // reference, MPC.cpp:175-176), the rest one more molecule
   ctx->mol_start.resize(n_rep);
@@ -1625,7 +1612,7 @@ int smpc_autotune(smpc_ctx* ctx, int cycles, char* report, int report_len) {
       int* var;
       const char* (*label)(int);
     } cats[4] = {{"fluid_bin", PH_BIN, smpc::bin_variant_count(), &ctx->var_bin, smpc::bin_variant_name},
-                 {"collide", PH_COLLIDE, smpc::collide_variant_count(), &ctx->var_col,
+                 {"collide", PH_COLLIDE, smpc::collide_shape_count(), &ctx->var_col,
                   smpc::collide_variant_name},
                  {"md_substeps", PH_MD, smpc::md_variant_count(), &ctx->var_md, smpc::md_variant_name},
                  {"pmd", PH_MD, smpc::pmd_variant_count(), &ctx->var_pmd, smpc::pmd_variant_name}};
