@@ -16,5 +16,9 @@ namespace smpc {
 int fluid_slots_per_tile(bool fp64) { return fp64 ? 2048 : 4096; }
 int temperature_cells_per_tile() { return 512; }
 int md_max_monomers() { return SMPC_MD_NT * SMPC_MD_MPT; }
+int profile_copies(size_t bins) { return bins <= 65536 ? PROF_COPIES : 1; }
+int stress_parts(int n_mono) {
+  return std::max(1, std::min(1024, (n_mono * STRESS_LANES + ANA_NT - 1) / ANA_NT));
+}
 int pmd_block_count(int n_beads) { return (n_beads + PMD_NT - 1) / PMD_NT; }
 }  // namespace smpc

@@ -181,12 +181,13 @@ template <>
 void launch_mono_stress<Real>(const RepInfo* reps, const RepDyn* dyn, int n_rep, const Real* mpos,
                               const Real* mvel, const int* nlist_t, const int* ncount,
                               int n_mono_total, int* const* rows, int max_nb,
-                              const int* bond_start, const int2* bonds, double* out,
-                              cudaStream_t st) {
+                              const int* bond_start, const int2* bonds, double* part,
+                              int n_part, double* out, cudaStream_t st) {
   if (n_rep == 0) return;
-  k_mono_stress<Real><<<n_rep, ANA_NT, 0, st>>>(reps, dyn, mpos, mvel, nlist_t, ncount,
-                                                n_mono_total, rows, max_nb, bond_start, bonds,
-                                                out);
+  k_mono_stress<Real><<<dim3(n_rep, n_part), ANA_NT, 0, st>>>(reps, dyn, mpos, mvel, nlist_t,
+                                                              ncount, n_mono_total, rows, max_nb,
+                                                              bond_start, bonds, part);
+  k_stress_reduce<Real><<<n_rep, 32, 0, st>>>(part, n_part, out);
 }
 
 template <>
@@ -256,12 +257,15 @@ template <>
 void launch_velocity_profile<Real>(const RepInfo* reps, const int2* rep_mols, const int2* mols,
                                    int rep, int slot_cap, const Real* rec, const Real* mpos,
                                    const Real* mvel, double delrx, double width, long long kx0,
-                                   int nx, long long ky0, int ny, double* c6, double* bins,
-                                   cudaStream_t st) {
-  k_profile_centre<Real><<<1, 1, 0, st>>>(rep_mols, mols, mpos, mvel, rep, c6);
-  if (slot_cap == 0) return;
-  k_velocity_profile<Real><<<(slot_cap + 255) / 256, 256, 0, st>>>(
-      reps, rep, rec, delrx, width, kx0, nx, ky0, ny, c6, bins);
+                                   int nx, long long ky0, int ny, double* c6, double* out,
+                                   double* bins, int n_copies, cudaStream_t st) {
+  k_profile_centre<Real><<<1, PROF_NT, 0, st>>>(rep_mols, mols, mpos, mvel, rep, c6);
+  constexpr int per_block = PROF_NT * PROF_RUN;
+  if (slot_cap > 0)
+    k_velocity_profile<Real><<<(slot_cap + per_block - 1) / per_block, PROF_NT, 0, st>>>(
+        reps, rep, rec, delrx, width, kx0, nx, ky0, ny, c6, bins, n_copies);
+  const int n = 3 * (nx + ny);
+  k_profile_reduce<Real><<<(n + 255) / 256, 256, 0, st>>>(bins, n, n_copies, out);
 }
 
 // Monomer state between the device's R4 records and x,y,z-interleaved double

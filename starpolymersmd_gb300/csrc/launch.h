@@ -135,7 +135,9 @@ template <typename R>
 void launch_velocity_profile(const RepInfo* reps, const int2* rep_mols, const int2* mols, int rep,
                              int slot_cap, const R* rec, const R* mpos, const R* mvel,
                              double delrx, double width, long long kx0, int nx, long long ky0,
-                             int ny, double* c6, double* bins, cudaStream_t st);
+                             int ny, double* c6, double* out, double* bins, int n_copies,
+                             cudaStream_t st);
+int profile_copies(size_t bins);  // copies of `bins` doubles that the profile's blocks add into
 
 // Solvent analyses (analysis.cuh); part: per-block partial sums.
 template <typename R>
@@ -157,7 +159,8 @@ template <typename R>
 void launch_mono_stress(const RepInfo* reps, const RepDyn* dyn, int n_rep, const R* mpos,
                         const R* mvel, const int* nlist_t, const int* ncount, int n_mono_total,
                         int* const* rows, int max_nb, const int* bond_start, const int2* bonds,
-                        double* out, cudaStream_t st);
+                        double* part, int n_part, double* out, cudaStream_t st);
+int stress_parts(int n_mono);  // blocks (partial sums) per replica of launch_mono_stress
 
 // Monomer state between the C ABI's x,y,z-interleaved doubles and the device
 // records (pos.w / vel.w keep mass and type): pos, vel, frc each 3M doubles, in

@@ -27,22 +27,48 @@ namespace smpc {
 constexpr int OBS_PER_REP = 16;
 constexpr int UNWRAP_NT = 256;  // threads (and beads per chunk) of k_unwrap_molecules
 
-// centre of molecule [b, e): unweighted mean position and velocity
-template <typename R>
+// A float as a double without a conversion instruction (those issue on the
+// narrow FP64 pipe): the exponent rebiased and the mantissa moved; zeros,
+// subnormals, infinities and NaNs take the conversion, out of line.
+static __device__ __noinline__ double to_d_special(float x) { return static_cast<double>(x); }
+__device__ __forceinline__ double to_d(float x) {
+  const uint32_t b = __float_as_uint(x), e = (b >> 23) & 255u;
+  if (e - 1u >= 254u) return to_d_special(x);
+  return __hiloint2double(static_cast<int>((b & 0x80000000u) |
+                                           (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)),
+                          static_cast<int>(b << 29));
+}
+__device__ __forceinline__ double to_d(double x) { return x; }
+
+// Centre of molecule [b, e), unweighted mean position and velocity, summed in
+// monomer order like the reference. The block stages the monomers in shared
+// memory, then six lanes add one component each: one thread that loaded and
+// added everything itself waited for memory at every monomer (185 us for 401
+// of them). c (shared) is valid after the caller's barrier.
+constexpr int CENTRE_CHUNK = 256;
+template <typename R, int NT>
 __device__ __forceinline__ void molecule_centre(const R* mpos, const R* mvel, int b, int e,
-                                                double* c) {
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int i = b; i < e; ++i) {
-    const R4<R> p = ld4_rw(mpos, i), v = ld4_rw(mvel, i);
-    s[0] += static_cast<double>(p.x);
-    s[1] += static_cast<double>(p.y);
-    s[2] += static_cast<double>(p.z);
-    s[3] += static_cast<double>(v.x);
-    s[4] += static_cast<double>(v.y);
-    s[5] += static_cast<double>(v.z);
+                                                R (*stage)[CENTRE_CHUNK], double* c) {
+  double s = 0.0;
+  for (int base = b; base < e; base += CENTRE_CHUNK) {
+    const int n = min(CENTRE_CHUNK, e - base);
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += NT) {
+      const R4<R> p = ld4_rw(mpos, base + i), v = ld4_rw(mvel, base + i);
+      stage[0][i] = p.x;
+      stage[1][i] = p.y;
+      stage[2][i] = p.z;
+      stage[3][i] = v.x;
+      stage[4][i] = v.y;
+      stage[5][i] = v.z;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+#pragma unroll 8
+      for (int i = 0; i < n; ++i) s += to_d(stage[threadIdx.x][i]);
+    }
   }
-  const double n = static_cast<double>(e - b);
-  for (int k = 0; k < 6; ++k) c[k] = s[k] / n;
+  if (threadIdx.x < 6) c[threadIdx.x] = s / static_cast<double>(e - b);
 }
 
 // x = A^-1 b for a symmetric positive-definite 3x3 A (LDL^T, no pivoting)
@@ -74,26 +100,46 @@ __device__ __forceinline__ double block_sum(double v, double* s_red) {
   return t;  // valid in thread 0
 }
 
-// K block sums at once, each with block_sum's order (so the same bits): one
-// shuffle pass over all K values, one exchange, thread k < K adds the warps'
-// partials of value k into out[k] (shared; valid in every thread on return).
-// s_red holds K * NT / 32 doubles.
+// K block sums at once into out[k] (shared; valid in every thread on return),
+// in a fixed order: every thread's values through shared memory, then warp w
+// sums values w, w + NT / 32, ...: NT / 32 partials per lane and one butterfly
+// per value (a butterfly per value in every warp took NT / 32 times the FP64
+// instructions). s_red holds K * NT doubles.
 template <int NT, int K>
 __device__ __forceinline__ void block_sum_n(double (&v)[K], double* s_red, double* out) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += __shfl_down_sync(0xFFFFFFFFu, v[k], o);
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) s_red[k * (NT / 32) + (threadIdx.x >> 5)] = v[k];
+  for (int k = 0; k < K; ++k) s_red[k * NT + threadIdx.x] = v[k];
   __syncthreads();
-  if (threadIdx.x < K) {
+  const int lane = threadIdx.x & 31;
+  for (int k = threadIdx.x >> 5; k < K; k += NT / 32) {
     double t = 0.0;
-    for (int w = 0; w < NT / 32; ++w) t += s_red[threadIdx.x * (NT / 32) + w];
-    out[threadIdx.x] = t;
+#pragma unroll
+    for (int w = 0; w < NT / 32; ++w) t += s_red[k * NT + 32 * w + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    if (lane == 0) out[k] = t;
   }
   __syncthreads();
+}
+
+// FP32 contexts: the same centre as a block reduction (7 us for 401 monomers,
+// with the kernel's launch).
+template <int NT>
+__device__ __forceinline__ void molecule_centre_f32(const float* mpos, const float* mvel, int b,
+                                                    int e, double* s_red, double* s_tot,
+                                                    double* c) {
+  double t[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = b + threadIdx.x; i < e; i += NT) {
+    const R4<float> p = ld4_rw(mpos, i), v = ld4_rw(mvel, i);
+    t[0] += to_d(p.x);
+    t[1] += to_d(p.y);
+    t[2] += to_d(p.z);
+    t[3] += to_d(v.x);
+    t[4] += to_d(v.y);
+    t[5] += to_d(v.z);
+  }
+  block_sum_n<NT, 6>(t, s_red, s_tot);
+  if (threadIdx.x < 6) c[threadIdx.x] = s_tot[threadIdx.x] / static_cast<double>(e - b);
 }
 
 // One CTA per molecule; mols[m] = global monomer range [x, y). mol_out[16 m
@@ -105,25 +151,15 @@ template <typename R, int NT>
 __global__ void __launch_bounds__(NT) k_mol_observables(const int2* mols, const R* mpos,
                                                         const R* mvel, double* mol_out) {
   __shared__ double s_c[6];
-  __shared__ double s_red[10 * (NT / 32)];
+  __shared__ double s_red[10 * NT];
   __shared__ double s_tot[10];
   const int2 mb = mols[blockIdx.x];
   const int n = mb.y - mb.x;
-  if (std::is_same<R, double>::value) {
-    if (threadIdx.x == 0) molecule_centre<R>(mpos, mvel, mb.x, mb.y, s_c);
+  if constexpr (std::is_same<R, double>::value) {
+    __shared__ R s_stage[6][CENTRE_CHUNK];
+    molecule_centre<R, NT>(mpos, mvel, mb.x, mb.y, s_stage, s_c);
   } else {
-    double c[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = mb.x + threadIdx.x; i < mb.y; i += NT) {
-      const R4<R> p = ld4_rw(mpos, i), v = ld4_rw(mvel, i);
-      c[0] += static_cast<double>(p.x);
-      c[1] += static_cast<double>(p.y);
-      c[2] += static_cast<double>(p.z);
-      c[3] += static_cast<double>(v.x);
-      c[4] += static_cast<double>(v.y);
-      c[5] += static_cast<double>(v.z);
-    }
-    block_sum_n<NT, 6>(c, s_red, s_tot);
-    if (threadIdx.x < 6) s_c[threadIdx.x] = s_tot[threadIdx.x] / static_cast<double>(n);
+    molecule_centre_f32<NT>(mpos, mvel, mb.x, mb.y, s_red, s_tot, s_c);
   }
   __syncthreads();
   // S = sum r r^T (6), angular momentum (3), sum m |u|^2
@@ -205,8 +241,8 @@ __global__ void k_obs_reduce(const int2* rep_mols, const double* mol_out, int n_
     for (int k = 0; k < 14; ++k) acc[k] += v[k];
     n_total += static_cast<long long>(v[14]);
   }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
+  // (one molecule: the other lanes' zeros change nothing)
+  for (int off = rm.y > 1 ? 16 : 0; off > 0; off >>= 1) {
 #pragma unroll
     for (int k = 0; k < 14; ++k) acc[k] += __shfl_xor_sync(FULL, acc[k], off);
     n_total += __shfl_xor_sync(FULL, n_total, off);
@@ -391,58 +427,147 @@ __global__ void __launch_bounds__(UNWRAP_NT)
   }
 }
 
+constexpr int PROF_NT = 128;   // threads per block of the profile kernels
+constexpr int PROF_RUN = 16;   // consecutive slots per thread of k_velocity_profile
+constexpr int PROF_COPIES = 128;  // copies of the bins that the blocks add into
+
 template <typename R>
-__global__ void k_profile_centre(const int2* rep_mols, const int2* mols, const R* mpos,
-                                 const R* mvel, int rep, double* c6) {
+__global__ void __launch_bounds__(PROF_NT) k_profile_centre(const int2* rep_mols, const int2* mols,
+                                                            const R* mpos, const R* mvel, int rep,
+                                                            double* c6) {
   const int2 rm = rep_mols[rep];
   if (rm.y == 0) {
-    for (int k = 0; k < 6; ++k) c6[k] = 0.0;
+    if (threadIdx.x < 6) c6[threadIdx.x] = 0.0;
     return;
   }
   const int2 mb = mols[rm.x];
-  molecule_centre<R>(mpos, mvel, mb.x, mb.y, c6);
+  if constexpr (std::is_same<R, double>::value) {
+    __shared__ R s_stage[6][CENTRE_CHUNK];
+    molecule_centre<R, PROF_NT>(mpos, mvel, mb.x, mb.y, s_stage, c6);
+  } else {
+    __shared__ double s_red[6 * PROF_NT], s_tot[6];
+    molecule_centre_f32<PROF_NT>(mpos, mvel, mb.x, mb.y, s_red, s_tot, c6);
+  }
 }
 
-// bins: x then y, 3 doubles per bin (sum v_x, sum v_y, count), zeroed by the host
+// floor(x / width), x / width rounded to a double as the reference's division
+// is: from x times the reciprocal, unless that is within 1e-9 of an integer
+// (or past 2^20, where its error could reach that), where the division decides.
+static __device__ __noinline__ long long profile_bin_div(double x, double width) {
+  return static_cast<long long>(floor(x / width));
+}
+__device__ __forceinline__ long long profile_bin(double x, double width, double inv) {
+  const double q = __dmul_rn(x, inv);
+  const double magic = 6755399441055744.0;           // 1.5 2^52: floor(q) in the low bits
+  const double t = __dadd_rd(q, magic);
+  const double r = __dsub_rn(q, __dsub_rn(t, magic));  // in [0, 1)
+  const long long k = __double2loint(t);
+  if (!(r > 1e-9 && r < 1.0 - 1e-9 && k > -(1 << 20) && k < (1 << 20)))
+    return profile_bin_div(x, width);
+  return k;
+}
+
+// One bin's running sums in a thread's registers.
+struct ProfAcc {
+  long long key;
+  double s0, s1;
+  int n;
+};
+__device__ __forceinline__ void prof_flush(ProfAcc& a, double* bins) {
+  if (a.n > 0) {
+    atomicAdd(bins + 3 * a.key, a.s0);
+    atomicAdd(bins + 3 * a.key + 1, a.s1);
+    atomicAdd(bins + 3 * a.key + 2, static_cast<double>(a.n));
+  }
+  a.s0 = a.s1 = 0.0;
+  a.n = 0;
+}
+__device__ __forceinline__ void prof_add(ProfAcc& even, ProfAcc& odd, long long k, long long n_bins,
+                                         double v0, double v1, double* bins) {
+  if (k < 0 || k >= n_bins) return;
+  ProfAcc& a = (k & 1) ? odd : even;
+  if (a.key != k) {
+    prof_flush(a, bins);
+    a.key = k;
+  }
+  a.s0 += v0;
+  a.s1 += v1;
+  ++a.n;
+}
+
+// bins: x then y, 3 doubles per bin (sum v_x, sum v_y, count), n_copies copies
+// zeroed by the host; block b adds into copy b mod n_copies. Every thread
+// walks PROF_RUN consecutive slots. The solvent is in cell order after a
+// collision, so a run meets a few bins only, two neighbouring ones per axis at
+// a time; their sums stay in registers (one pair for even bins, one for odd)
+// and go out when the bin changes. One atomic per particle and sum onto the
+// few hundred addresses took 1015 us for 1.25 M particles; this takes 124 with
+// the slots in id order, where every particle changes the bin. Wraps and bins
+// are decided without divisions.
 template <typename R>
-__global__ void k_velocity_profile(const RepInfo* reps, int rep, const R* rec, double delrx,
-                                   double width, long long kx0, int nx, long long ky0, int ny,
-                                   const double* c6, double* bins) {
+__global__ void __launch_bounds__(PROF_NT)
+    k_velocity_profile(const RepInfo* reps, int rep, const R* rec, double delrx, double width,
+                       long long kx0, int nx, long long ky0, int ny, const double* c6,
+                       double* bins, int n_copies) {
   const RepInfo& ri = reps[rep];
+  const int i0 = (blockIdx.x * PROF_NT + threadIdx.x) * PROF_RUN;
+  const int i1 = min(i0 + PROF_RUN, ri.slot_cap);
+  double* bx = bins + static_cast<size_t>(blockIdx.x % n_copies) * 3 * static_cast<size_t>(nx + ny);
+  double* by = bx + 3 * static_cast<size_t>(nx);
+  const double c0 = c6[0], c1 = c6[1], cv0 = c6[3], cv1 = c6[4];
+  const double Lx = ri.L[0], Ly = ri.L[1], inv = 1.0 / width;
+  const double jump = __dmul_rn(ri.shear, Ly);
+  const bool sheared = ri.shear != 0.0;
+  long long lo[2], half[2], far[2];
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {  // as make_geo: L/2 (1 - 2^-50), L/2, 1.5 L (1 - 2^-50)
+    const double h = static_cast<double>(ri.L[d]) * 0.5;
+    lo[d] = __double_as_longlong(h * (1.0 - 0x1.0p-50));
+    half[d] = __double_as_longlong(h);
+    far[d] = __double_as_longlong(3.0 * h * (1.0 - 0x1.0p-50));
+  }
+  ProfAcc xe{0, 0.0, 0.0, 0}, xo{1, 0.0, 0.0, 0}, ye{0, 0.0, 0.0, 0}, yo{1, 0.0, 0.0, 0};
+  for (int i = i0; i < i1; ++i) {
+    const size_t s = static_cast<size_t>(ri.slot_base) + i;
+    const R4<R> p = ld_pos(rec, s), v = ld_vel(rec, s);
+    if (slot_id(p.w) == SLOT_EMPTY) continue;
+    double x0 = to_d(p.x) - c0, x1 = to_d(p.y) - c1;
+    double v0 = to_d(v.x) - cv0;
+    const double v1 = to_d(v.y) - cv1;
+    const long long a0 = __double_as_longlong(x0) & 0x7FFFFFFFFFFFFFFFll;
+    const long long a1 = __double_as_longlong(x1) & 0x7FFFFFFFFFFFFFFFll;
+    if (a0 >= lo[0] || a1 >= lo[1]) {  // MPC::LEBC(pos, vel) (MPC.cpp:431-439), MPC::wrap(pos)
+      if (sheared) {
+        const double cy = image_d(x1, Ly, lo[1], half[1], far[1]);
+        x0 = wrap_d(x0, Lx, lo[0], half[0], far[0]);
+        if (cy != 0.0) {
+          x0 = __dsub_rn(x0, __dmul_rn(cy, delrx));
+          x1 = __dsub_rn(x1, __dmul_rn(Ly, cy));
+          v0 = __dsub_rn(v0, __dmul_rn(cy, jump));
+        }
+        x0 = wrap_d(x0, Lx, lo[0], half[0], far[0]);
+      } else {
+        x0 = wrap_d(x0, Lx, lo[0], half[0], far[0]);
+        x1 = wrap_d(x1, Ly, lo[1], half[1], far[1]);
+      }
+    }
+    prof_add(xe, xo, profile_bin(x0, width, inv) - kx0, nx, v0, v1, bx);
+    prof_add(ye, yo, profile_bin(x1, width, inv) - ky0, ny, v0, v1, by);
+  }
+  prof_flush(xe, bx);
+  prof_flush(xo, bx);
+  prof_flush(ye, by);
+  prof_flush(yo, by);
+}
+
+// The copies of the bins, in order, into out.
+template <typename R>  // R: the precision of the instantiating unit (one copy per unit)
+__global__ void k_profile_reduce(const double* bins, int n, int n_copies, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ri.slot_cap) return;
-  const size_t s = static_cast<size_t>(ri.slot_base) + i;
-  const R* p = rec + 8 * s;
-  if (slot_id(p[3]) == SLOT_EMPTY) return;
-  double x0 = static_cast<double>(p[0]) - c6[0], x1 = static_cast<double>(p[1]) - c6[1],
-         x2 = static_cast<double>(p[2]) - c6[2];
-  double v0 = static_cast<double>(p[4]) - c6[3], v1 = static_cast<double>(p[5]) - c6[4];
-  const double Lx = ri.L[0], Ly = ri.L[1], Lz = ri.L[2];
-  if (ri.shear != 0.0) {  // MPC::LEBC(pos, vel) (MPC.cpp:431-439)
-    const double cy = round(x1 / Ly);
-    x0 -= Lx * round(x0 / Lx);
-    x0 -= cy * delrx;
-    x0 -= Lx * round(x0 / Lx);
-    x1 -= Ly * cy;
-    x2 -= Lz * round(x2 / Lz);
-    v0 -= cy * ri.shear * Ly;
-  } else {  // MPC::wrap(pos) (MPC.cpp:473-478)
-    x0 -= round(x0 / Lx) * Lx;
-    x1 -= round(x1 / Ly) * Ly;
-  }
-  const long long kx = static_cast<long long>(floor(x0 / width)) - kx0;
-  const long long ky = static_cast<long long>(floor(x1 / width)) - ky0;
-  if (kx >= 0 && kx < nx) {
-    atomicAdd(bins + 3 * kx, v0);
-    atomicAdd(bins + 3 * kx + 1, v1);
-    atomicAdd(bins + 3 * kx + 2, 1.0);
-  }
-  if (ky >= 0 && ky < ny) {
-    double* b = bins + 3 * static_cast<size_t>(nx);
-    atomicAdd(b + 3 * ky, v0);
-    atomicAdd(b + 3 * ky + 1, v1);
-    atomicAdd(b + 3 * ky + 2, 1.0);
-  }
+  if (i >= n) return;
+  double t = 0.0;
+  for (int c = 0; c < n_copies; ++c) t += bins[static_cast<size_t>(c) * n + i];
+  out[i] = t;
 }
 
 }  // namespace smpc

@@ -103,7 +103,8 @@ struct smpc_ctx {
   size_t ana_part_cap = 0;
   double* d_vacf_ring = nullptr;
   int** d_rows_by_rep = nullptr;  // each replica's periodic Verlet rows, or null
-  double* d_stress = nullptr;     // 12 per replica
+  double* d_stress = nullptr;     // 12 per replica, then 12 per partial sum
+  int stress_parts = 1;           // partial sums per replica
   int vacf_rep = -1, vacf_np = 0, vacf_entries = 0;
   uint64_t vacf_samples = 0, vacf_calcs = 0;
   std::vector<double> vacf_sum;
@@ -962,7 +963,9 @@ int create_periodic_md(smpc_ctx* ctx) {
     CU(dalloc(&ctx->d_rows_by_rep, rows.size()));
     CU(cudaMemcpy(ctx->d_rows_by_rep, rows.data(), rows.size() * sizeof(int*),
                   cudaMemcpyHostToDevice));
-    CU(dalloc(&ctx->d_stress, 12 * static_cast<size_t>(ctx->n_rep)));
+    for (const RepInfo& ri : ctx->reps)
+      ctx->stress_parts = std::max(ctx->stress_parts, smpc::stress_parts(ri.n_mono));
+    CU(dalloc(&ctx->d_stress, 12 * static_cast<size_t>(ctx->n_rep) * (1 + ctx->stress_parts)));
   }
   if (!ctx->pmd.empty()) {
     CU(cudaMalloc(&ctx->d_pamphi, M));
@@ -1899,13 +1902,15 @@ void mol_observables_t(smpc_ctx* ctx) {
 template <typename R>
 void velocity_profile_t(smpc_ctx* ctx, int rep, double width, long long kx0, int n_x,
                         long long ky0, int n_y) {
+  const size_t nb = 3 * static_cast<size_t>(n_x + n_y);
   const R *p, *v;
   observed_monomers<R>(ctx, &p, &v);
   smpc::launch_velocity_profile<R>(ctx->d_reps, ctx->d_rep_mols, ctx->d_mols, rep,
                                    ctx->reps[rep].slot_cap,
                                    static_cast<const R*>(ctx->d_rec[ctx->cur]), p, v,
                                    ctx->dyn[rep].delrx, width, kx0, n_x, ky0, n_y, ctx->d_c6,
-                                   ctx->d_prof, ctx->st);
+                                   ctx->d_prof, ctx->d_prof + nb, smpc::profile_copies(nb),
+                                   ctx->st);
 }
 }  // namespace
 
@@ -1986,16 +1991,17 @@ int smpc_velocity_profile(smpc_ctx* ctx, int rep, double width, double* x_out, i
     return fail(ctx, SMPC_E_ARG, "profile needs " + std::to_string(need_x) + " x bins and " +
                                      std::to_string(need_y) + " y bins");
   cudaSetDevice(ctx->device);
-  const size_t nb = 3 * static_cast<size_t>(n_x + n_y);
-  if (nb > ctx->prof_cap) {
+  // the result, then the copies that the blocks add into
+  const size_t nb = 3 * static_cast<size_t>(n_x + n_y), nc = nb * smpc::profile_copies(nb);
+  if (nb + nc > ctx->prof_cap) {
     CU(cudaStreamSynchronize(ctx->st));
     if (ctx->d_prof) cudaFree(ctx->d_prof);
     ctx->d_prof = nullptr;
     ctx->prof_cap = 0;
-    CU(dalloc(&ctx->d_prof, nb));
-    ctx->prof_cap = nb;
+    CU(dalloc(&ctx->d_prof, nb + nc));
+    ctx->prof_cap = nb + nc;
   }
-  CU(cudaMemsetAsync(ctx->d_prof, 0, nb * sizeof(double), ctx->st));
+  CU(cudaMemsetAsync(ctx->d_prof + nb, 0, nc * sizeof(double), ctx->st));
   if (ctx->total_mono > 0 && !ctx->md_ready && !ctx->pmd.empty())
     return fail(ctx, SMPC_E_STATE, "smpc_init_md not called (bonds make periodic molecules whole)");
   if (ctx->opt.precision == SMPC_FP64)
@@ -2092,7 +2098,8 @@ int smpc_pressure_tensor_all(smpc_ctx* ctx, double* out) {
                                      static_cast<const double*>(ctx->d_mvel), ctx->d_nlist,
                                      ctx->d_ncount, static_cast<int>(ctx->total_mono),
                                      ctx->d_rows_by_rep, ctx->max_nb, ctx->d_bond_start,
-                                     ctx->d_bonds, ctx->d_stress, ctx->st);
+                                     ctx->d_bonds, ctx->d_stress + 12 * ctx->n_rep, ctx->stress_parts,
+                                     ctx->d_stress, ctx->st);
   } else {
     smpc::launch_kinetic_tensor<float>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps,
                                        static_cast<const float*>(ctx->d_rec[ctx->cur]),
@@ -2102,7 +2109,8 @@ int smpc_pressure_tensor_all(smpc_ctx* ctx, double* out) {
                                     static_cast<const float*>(ctx->d_mvel), ctx->d_nlist,
                                     ctx->d_ncount, static_cast<int>(ctx->total_mono),
                                     ctx->d_rows_by_rep, ctx->max_nb, ctx->d_bond_start,
-                                    ctx->d_bonds, ctx->d_stress, ctx->st);
+                                    ctx->d_bonds, ctx->d_stress + 12 * ctx->n_rep, ctx->stress_parts,
+                                     ctx->d_stress, ctx->st);
   }
   CU(cudaGetLastError());
   std::vector<double> part(6 * static_cast<size_t>(ctx->n_bin_tiles));
