@@ -99,6 +99,7 @@ struct MdSplit {
   cudaStream_t st2;
   cudaEvent_t fork, join;
   int n_big;
+  int max_bond_ends[2];  // of any non-periodic replica (two per bond): up to 512 beads; larger
   int cluster;  // > 0: non-periodic MD on clusters of this many CTAs per replica (k_md_cluster)
 };
 // Largest cluster size (16 or 8) at which k_md_cluster<R> can run on the

@@ -93,6 +93,25 @@ __device__ __forceinline__ float pair_force<float>(int pot, bool bb, float r2, f
   return 0.0f;
 }
 
+// pair_force<float> without a branch around the arithmetic (zero out of range
+// and where `use` is false)
+__device__ __forceinline__ float pair_force_all(int pot, bool bb, float r2, float lambda, bool use) {
+  if (pot == POT_REF4824) {
+    const bool core = r2 < 1.0594631f, in = use && (core || (bb && r2 < 2.25f));
+    const float rm2 = __frcp_rn(in ? r2 : 1.0f);
+    float rm24 = rm2 * rm2 * rm2;
+    rm24 *= rm24;
+    rm24 *= rm24;
+    const float f = 192.0f * rm2 * rm24 * (rm24 - 0.5f);
+    return in ? (core ? f : lambda * f) : 0.0f;
+  }
+  const bool core = r2 < 1.2599210498948732f, in = use && (core || (bb && r2 < 6.25f));
+  const float rm2 = __frcp_rn(in ? r2 : 1.0f);
+  const float rm6 = rm2 * rm2 * rm2;
+  const float f = 48.0f * rm2 * rm6 * (rm6 - 0.5f);
+  return in ? (core ? f : lambda * f) : 0.0f;
+}
+
 template <typename R>
 __device__ __forceinline__ R pair_pot(int pot, bool bb, R r2, R lambda) {
   if (pot == POT_REF4824) {
@@ -378,15 +397,16 @@ __device__ __forceinline__ int md_warp_scan(int v) {
   return v;
 }
 
-// Beads in bucket order, each bucket in ascending bead order (the order the
-// sorted chains give), as a counting sort: one warp ranks the beads within
-// their buckets in bead order, 32 at a time (__match_any_sync groups a
-// batch's beads by bucket), the block scans the counts, and every bead goes
-// to its bucket's start plus its rank. s_bkt[j]: bucket of bead j, set by
-// the caller (the rank is packed beside it: bucket | rank << 11);
-// s_start[MD_BUCKETS + 1]: bucket starts; s_sorted[k]: the k-th bead. Ends
-// with the block synchronised. A cell's members are then a contiguous run to
-// scan, not a chain of dependent loads.
+// Beads in bucket order, each bucket in ascending bead order, as a counting
+// sort: atomics count the buckets and give every bead some slot of its bucket,
+// a block scan gives the bucket starts, the beads go to their slots, and each
+// then counts the smaller ones among its bucket's few members, which gives its
+// place whatever order the atomics ran in. (One warp that ranked the beads 32
+// at a time in order took 9,000 cycles for 401 beads; this takes a quarter.)
+// s_bkt[j]: bucket of bead j, set by the caller (the place is packed beside it:
+// bucket | place << 11); s_start[MD_BUCKETS + 1]: bucket starts; s_sorted[k]:
+// the k-th bead. Ends with the block synchronised. A cell's members are then a
+// contiguous run to scan, not a chain of dependent loads.
 template <int NT>
 __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, int* s_sorted) {
   static_assert(MD_BUCKETS == 2048, "11-bit bucket field");
@@ -394,21 +414,9 @@ __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, 
   constexpr int PER = MD_BUCKETS / NT;
   for (int t = threadIdx.x; t <= MD_BUCKETS; t += NT) s_start[t] = 0;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const unsigned lane = threadIdx.x;
-    for (int j0 = 0; j0 < n; j0 += 32) {
-      const int j = j0 + static_cast<int>(lane);
-      const int bk = j < n ? s_bkt[j] : -1 - static_cast<int>(lane);
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, bk);
-      const int leader = __ffs(peers) - 1;
-      int base = 0;
-      if (j < n && static_cast<int>(lane) == leader) {
-        base = s_start[bk];
-        s_start[bk] = base + __popc(peers);
-      }
-      base = __shfl_sync(0xFFFFFFFFu, base, leader);
-      if (j < n) s_bkt[j] = bk | ((base + __popc(peers & ((1u << lane) - 1u))) << 11);
-    }
+  for (int j = threadIdx.x; j < n; j += NT) {
+    const int bk = s_bkt[j];
+    s_bkt[j] = bk | (atomicAdd(s_start + bk, 1) << 11);
   }
   __syncthreads();
   {  // exclusive scan of the counts: PER consecutive buckets per thread
@@ -425,6 +433,16 @@ __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, 
 #pragma unroll
     for (int u = 0; u < PER; ++u) { s_start[PER * threadIdx.x + u] = run; run += c[u]; }
     if (threadIdx.x == NT - 1) s_start[MD_BUCKETS] = run;
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < n; j += NT)
+    s_sorted[s_start[s_bkt[j] & 2047] + (s_bkt[j] >> 11)] = j;
+  __syncthreads();
+  for (int j = threadIdx.x; j < n; j += NT) {
+    const int bk = s_bkt[j] & 2047;
+    int place = 0;
+    for (int k = s_start[bk]; k < s_start[bk + 1]; ++k) place += s_sorted[k] < j ? 1 : 0;
+    s_bkt[j] = bk | (place << 11);
   }
   __syncthreads();
   for (int j = threadIdx.x; j < n; j += NT)
@@ -815,6 +833,509 @@ __device__ __noinline__ void md_bead_forces_lists(const MdArgs& a, int b, int i,
   F[2] = F2;
 }
 
+
+// ---------------------------------------------------------------------------
+// The FP32 substeps of one replica per CTA with the lists in shared memory
+// (no Lowe-Andersen; at most NT beads). Results are those of k_md_substeps
+// with one bead per thread and up to KMAX lanes per bead, to the last bit:
+// the Verlet lists, their order and the order of every sum are the same.
+//
+//  * Lists: each thread keeps its share of its bead's list in shared memory,
+//    without the pairs that cannot come into range before the next rebuild:
+//    beads that do not attract act on each other up to 1.12 only, and their
+//    pairs beyond 1.12 + skin carry exactly zero force until then. About a
+//    third of the entries are left, and none is read from L2 in a substep.
+//  * Rebuilds: a warp takes one occupied cell at a time. All beads of a cell
+//    have the same 27 neighbour cells, so the warp lists those cells' members
+//    once, 32 candidates at a time, and tests them against every bead of the
+//    cell; ballots keep the order (cells, then beads, ascending) in which one
+//    lane walking alone would find them. That walk took 78,000 cycles for 121
+//    beads and 97,000 for 401, seven tenths of the kernel's time at the one
+//    rebuild in five substeps of a relaxed star; this takes 14,000 and 39,000.
+//  * Bonds are in shared memory; every bond end is computed by a thread of its
+//    own and added in order by its bead's lead lane (a star's core has one
+//    bond per arm).
+//  * The half-kick increment is computed once per force evaluation, and
+//    positions alternate between two buffers: two barriers per substep.
+constexpr unsigned short MD_NO_ENTRY = 0xFFFFu;
+// Bond ends of a replica (two per bond) that fit: a star of NT beads has NT - 1 bonds.
+constexpr int md_fast_bonds(int nt) { return 2 * nt; }
+template <int NT, int ROWS>
+struct MdFastSmem {
+  static constexpr int BONDS = md_fast_bonds(NT);
+  float4 pos[2][NT];              // positions, by substep parity
+  float4 ref[NT];                 // positions at the last list build
+  float4 bf[BONDS];               // per bond end: the bond's vector and force factor
+  int head[MD_BUCKETS + 1];       // bucket starts in sorted
+  int sorted[NT];                 // beads by bucket
+  int bucket[NT];                 // bucket of each bead
+  int ckey[NT];                   // cell of each bead
+  unsigned short ent[ROWS * NT];  // entry t of thread T at t NT + T: partner | attracting << 15
+  unsigned short n_ent[NT];
+  unsigned short cells[NT];       // place in sorted of every occupied cell's first bead
+  unsigned short bond[BONDS];     // per bond end: partner | anchor bond << 15
+  unsigned short bead[BONDS];     // and the bead itself
+  unsigned short bstart[NT + 2];
+  unsigned char amphi[NT];
+  int n_cells, next_cell;
+  float core_ref[3];
+};
+// Squared distance at the list build up to which a pair is kept: its cut-off
+// plus the skin, which two beads use up together before a rebuild, and a
+// margin far above FP32 rounding.
+__device__ __forceinline__ float md_keep_r2(int pot, bool bb, float skin) {
+  const float cut2 = pot == POT_REF4824 ? (bb ? 2.25f : 1.0594631f)
+                                        : (bb ? 6.25f : 1.2599210498948732f);
+  const float r = sqrtf(cut2) + fmaxf(skin, 0.0f) + 1e-3f;
+  return r * r;
+}
+
+// FENE bond of a bead at x with one at y: its vector d and force factor.
+__device__ __forceinline__ float md_bond_f32(const MdArgs& a, int pot, bool anch, float4 y,
+                                             const float* x, float* d, float* r2_out, int gi,
+                                             int gj) {
+  d[0] = y.x - x[0];
+  d[1] = y.y - x[1];
+  d[2] = y.z - x[2];
+  float r2 = (d[0] * d[0] + d[1] * d[1]) + d[2] * d[2];
+  if (pot == POT_REF4824) {
+    // reference FENE: beyond R0 the force changes sign (Potentials.h:24-55)
+    if (r2 >= (anch ? 20.25f : 2.25f))
+      raise_error(a.err, ERR_FENE, static_cast<uint32_t>(gi), static_cast<uint32_t>(gj));
+  } else {
+    // 12-6 preset: FENE argument capped at 0.98 R0^2 (finite, restoring)
+    const float cap = (anch ? 20.25f : 2.25f) * 0.98f;
+    if (r2 > cap) r2 = cap;
+  }
+  *r2_out = r2;
+  return fene_force<float>(anch, r2);
+}
+
+// Forces on bead i from its list in global memory, every (1 << lk)-th entry
+// from sub, and on the lead lane its bonds (a block whose shares of the lists
+// outgrow the shared memory).
+static __device__ __noinline__ void md_bead_forces_global(const MdArgs& a, int b, int i, int sub,
+                                                          int lk, const float4* pos,
+                                                          const unsigned char* amphi, int pot,
+                                                          float lambda, bool want_epot, float* F,
+                                                          double* epot) {
+  const float4 xi = pos[i];
+  const float x[3] = {xi.x, xi.y, xi.z};
+  float F0 = 0.0f, F1 = 0.0f, F2 = 0.0f;
+  const bool ai = amphi[i] != 0;
+  const int cnt = a.ncount[b + i];
+  const int* nl = a.nlist + b + i;
+  const size_t stride = static_cast<size_t>(a.n_mono_total);
+  for (int q = sub; q < cnt; q += 1 << lk) {
+    const int j = nl[static_cast<size_t>(q) * stride] - b;
+    const float4 y = pos[j];
+    const float d0 = y.x - x[0], d1 = y.y - x[1], d2 = y.z - x[2];
+    const float r2 = (d0 * d0 + d1 * d1) + d2 * d2;
+    const bool bb = ai && amphi[j] != 0;
+    const float fa = pair_force<float>(pot, bb, r2, lambda);
+    F0 -= d0 * fa;
+    F1 -= d1 * fa;
+    F2 -= d2 * fa;
+    if (want_epot) *epot += md_pair_epot<float>(pot, bb, r2, lambda);
+  }
+  if (sub == 0)
+    for (int e = a.bond_start[b + i]; e < a.bond_start[b + i + 1]; ++e) {
+      const int2 bd = a.bonds[e];
+      float d[3], r2;
+      const float fa = md_bond_f32(a, pot, bd.y != 0, pos[bd.x - b], x, d, &r2, b + i, bd.x);
+      F0 -= d[0] * fa;
+      F1 -= d[1] * fa;
+      F2 -= d[2] * fa;
+      if (want_epot) *epot += md_fene_epot<float>(bd.y != 0, r2);
+    }
+  F[0] = F0;
+  F[1] = F1;
+  F[2] = F2;
+}
+
+template <int NT, int KMAX, int ROWS>
+__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1)
+    k_md_fast(MdArgs a, float* mpos, float* mvel, float* mfrc, float* mver) {
+  static_assert(NT <= 1024, "list entries hold 10-bit partners");
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  MdFastSmem<NT, ROWS>& S = *reinterpret_cast<MdFastSmem<NT, ROWS>*>(s_dyn);
+  __shared__ double s_red[NT / 32];
+  const int r = a.order ? a.order[blockIdx.x] : static_cast<int>(blockIdx.x);
+  const RepInfo& ri = a.reps[r];
+  const int n = ri.n_mono;
+  if (n == 0 || (ri.flags & REP_PERIODIC_MD)) return;  // periodic boxes: pmd_kernels.cuh
+  int lk = 0;  // log2 of the lanes per bead
+  while ((2 << lk) <= KMAX && (n << (lk + 1)) <= NT) ++lk;
+  const int kmask = (1 << lk) - 1;
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
+  const int sub = tid & kmask;
+  const int i = tid >> lk;  // bead of this lane
+  const bool mine = i < n, lead = sub == 0;
+  const int b = ri.mono_base;
+  const float dt = static_cast<float>(ri.md_dt);
+  const float dth = dt * 0.50f;
+  const float lambda = static_cast<float>(ri.lambda);
+  const float rv = static_cast<float>(ri.r_verlet);
+  const float rv2 = rv * rv;
+  const float skin = rv - static_cast<float>(ri.r_cut);
+  const float lim = skin * 0.5f;
+  const int pot = ri.potential;
+  const float keep_bb = md_keep_r2(pot, true, skin), keep_aa = md_keep_r2(pot, false, skin);
+  const unsigned long long md_step0 = a.dyn[r].md_step;  // thread 0 adds n_steps at the end
+
+  float x[3] = {0, 0, 0}, v[3] = {0, 0, 0}, f[3] = {0, 0, 0}, fk[3] = {0, 0, 0}, xv[3] = {0, 0, 0},
+        m = 1.0f;
+  auto increment = [&]() {  // f / m dt / 2 of the half kicks (Thermostat_None.cpp:22,34)
+    for (int d = 0; d < 3; ++d) fk[d] = a.andersen ? f[d] * (dth / m) : (f[d] / m) * dth;
+  };
+  if (mine) {
+    const R4<float> p = ld4_rw(mpos, b + i), vv = ld4_rw(mvel, b + i), ff = ld4_rw(mfrc, b + i),
+                    pv = ld4_rw(mver, b + i);
+    x[0] = p.x; x[1] = p.y; x[2] = p.z; m = p.w;
+    v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
+    f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
+    xv[0] = pv.x; xv[1] = pv.y; xv[2] = pv.z;
+    increment();
+    if (lead) {
+      S.amphi[i] = static_cast<unsigned char>(static_cast<int>(vv.w) & 1);
+      S.pos[0][i] = make_float4(p.x, p.y, p.z, 0.0f);
+      S.ref[i] = make_float4(pv.x, pv.y, pv.z, 0.0f);
+      if (i == 0) {  // the core's position at the last list build
+        S.core_ref[0] = pv.x; S.core_ref[1] = pv.y; S.core_ref[2] = pv.z;
+      }
+    }
+  }
+  const int bond0 = a.bond_start[b], n_bond = a.bond_start[b + n] - bond0;  // <= md_fast_bonds(NT)
+  {
+    const int e0 = bond0;
+    for (int j = tid; j <= n; j += NT) {
+      const int s0 = a.bond_start[b + j] - e0;
+      S.bstart[j] = static_cast<unsigned short>(s0);
+      if (j < n)
+        for (int e = s0; e < a.bond_start[b + j + 1] - e0; ++e)
+          S.bead[e] = static_cast<unsigned short>(j);
+    }
+    for (int e = tid; e < n_bond; e += NT) {
+      const int2 bd = a.bonds[e0 + e];
+      S.bond[e] = static_cast<unsigned short>((bd.x - b) | (bd.y != 0 ? 0x8000 : 0));
+    }
+  }
+  int n_ent = -1;        // entries of this thread (-1: to be taken from the global lists)
+  bool fits = true;      // every thread's entries fit
+  int rebuilds = 0;
+  double epot = 0.0;
+  const int total_steps = a.n_steps > 0 ? a.n_steps : 1;
+  for (int step = 0; step < total_steps; ++step) {
+    float4* const pos = S.pos[step & 1];
+    bool over = step == 0 && a.force_rebuild;
+    if (a.n_steps > 0) {
+      // kick + drift (Thermostat_None.cpp:22-27)
+      if (mine) {
+        for (int d = 0; d < 3; ++d) {
+          v[d] += fk[d];
+          x[d] += v[d] * dt;
+        }
+        if (lead) pos[i] = make_float4(x[0], x[1], x[2], 0.0f);
+        if (!a.core_relative) {  // Box::check_VerletLists (Box.cpp:182-194)
+          const float d0 = x[0] - xv[0], d1 = x[1] - xv[1], d2 = x[2] - xv[2];
+          over = over || sqrtf((d0 * d0 + d1 * d1) + d2 * d2) > lim;
+        }
+      }
+      if (a.core_relative) {
+        // displacements relative to the core's (see k_md_substeps)
+        __syncthreads();
+        if (mine) {
+          const float4 c = pos[0];
+          const float c0 = c.x - S.core_ref[0], c1 = c.y - S.core_ref[1], c2 = c.z - S.core_ref[2];
+          const float d0 = x[0] - xv[0] - c0, d1 = x[1] - xv[1] - c1, d2 = x[2] - xv[2] - c2;
+          over = over || (d0 * d0 + d1 * d1) + d2 * d2 > lim * lim;
+        }
+      }
+    }
+    if (__syncthreads_or(over)) {
+      // Verlet lists: every other bead within r_verlet (Box.cpp:146-179), found
+      // through a hashed grid of side r_verlet
+      ++rebuilds;
+      const float inv_rv = 1.0f / rv;
+      for (int j = tid; j < n; j += NT) {
+        const float4 p = pos[j];
+        const int cx = static_cast<int>(floorf(p.x * inv_rv)),
+                  cy = static_cast<int>(floorf(p.y * inv_rv)),
+                  cz = static_cast<int>(floorf(p.z * inv_rv));
+        S.ckey[j] = md_cell_key(cx, cy, cz);
+        S.bucket[j] = md_bucket(cx, cy, cz);
+        S.ref[j] = p;
+      }
+      if (tid == 0) {
+        S.n_cells = S.next_cell = 0;
+        S.core_ref[0] = pos[0].x; S.core_ref[1] = pos[0].y; S.core_ref[2] = pos[0].z;
+      }
+      xv[0] = x[0]; xv[1] = x[1]; xv[2] = x[2];
+      __syncthreads();
+      md_bucket_sort<NT>(n, S.bucket, S.head, S.sorted);
+      // the occupied cells, each by the place of its first bead
+      for (int p = tid; p < n; p += NT) {
+        const int key = S.ckey[S.sorted[p]];
+        const int bk = S.bucket[S.sorted[p]] & (MD_BUCKETS - 1);
+        bool first = true;
+        for (int q = S.head[bk]; q < p && first; ++q) first = S.ckey[S.sorted[q]] != key;
+        if (first) S.cells[atomicAdd(&S.n_cells, 1)] = static_cast<unsigned short>(p);
+      }
+      __syncthreads();
+      const unsigned lt = (1u << lane) - 1u;
+      for (;;) {
+        int cell = 0;
+        if (lane == 0) cell = atomicAdd(&S.next_cell, 1);
+        cell = __shfl_sync(FULL, cell, 0);
+        if (cell >= S.n_cells) break;
+        const int p0 = S.cells[cell];
+        const int j0 = S.sorted[p0], key0 = S.ckey[j0];
+        const float4 c = pos[j0];
+        const int cx = static_cast<int>(floorf(c.x * inv_rv)),
+                  cy = static_cast<int>(floorf(c.y * inv_rv)),
+                  cz = static_cast<int>(floorf(c.z * inv_rv));
+        // lanes 0..26: one neighbour cell each
+        int want = 0, start = 0, cnt = 0;
+        if (lane < 27) {
+          const int tx = cx + lane % 3 - 1, ty = cy + (lane / 3) % 3 - 1, tz = cz + lane / 9 - 1;
+          want = md_cell_key(tx, ty, tz);
+          const int bk = md_bucket(tx, ty, tz);
+          start = S.head[bk];
+          cnt = S.head[bk + 1] - start;
+        }
+        const int incl = md_warp_scan(cnt);
+        const int excl = incl - cnt;
+        const int total = __shfl_sync(FULL, incl, 31);
+        const int pend = S.head[md_bucket(cx, cy, cz) + 1];
+        for (int pb = p0; pb < pend;) {
+          // up to 32 beads of the cell: lane g holds the g-th and its counts
+          int mine_i = -1, acc = 0, kept = 0, n_b = 0, pn = pb;
+          for (; pn < pend && n_b < 32; pn += 32) {
+            const int jj = pn + lane < pend ? S.sorted[pn + lane] : -1;
+            unsigned mk = __ballot_sync(FULL, jj >= 0 && S.ckey[jj < 0 ? 0 : jj] == key0);
+            if (n_b + __popc(mk) > 32) break;  // the rest in another pass over the candidates
+            while (mk) {
+              const int src = __ffs(mk) - 1;
+              const int id = __shfl_sync(FULL, jj, src);
+              if (lane == n_b) mine_i = id;
+              ++n_b;
+              mk &= mk - 1;
+            }
+          }
+          pb = pn;
+          for (int k0 = 0; k0 < total; k0 += 32) {
+            const int k = k0 + lane;
+            int L = 0;  // the cell lane whose range [excl, incl) holds k
+#pragma unroll
+            for (int st = 16; st > 0; st >>= 1) {
+              const int e = __shfl_sync(FULL, excl, L + st);
+              if (L + st < 27 && e <= k) L += st;
+            }
+            const int w = __shfl_sync(FULL, want, L);
+            const int at = __shfl_sync(FULL, start, L) + k - __shfl_sync(FULL, excl, L);
+            int j = -1;
+            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+            bool aj = false;
+            if (k < total) {
+              j = S.sorted[at];
+              if (S.ckey[j] != w) j = -1;
+              if (j >= 0) {
+                y = pos[j];
+                aj = S.amphi[j] != 0;
+              }
+            }
+            for (int g = 0; g < n_b; ++g) {
+              const int id = __shfl_sync(FULL, mine_i, g);
+              const float4 xi = pos[id];
+              const float d0 = y.x - xi.x, d1 = y.y - xi.y, d2 = y.z - xi.z;
+              const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d0, d0, __fmul_rn(d1, d1)));
+              const bool in = j >= 0 && j != id && r2 <= rv2;
+              const unsigned mk = __ballot_sync(FULL, in);
+              if (mk == 0) continue;
+              const int q = __shfl_sync(FULL, acc, g) + __popc(mk & lt);
+              const bool bb = aj && S.amphi[id] != 0;
+              const bool put = in && q < a.max_nb;
+              if (put)
+                a.nlist[static_cast<size_t>(q) * a.n_mono_total + b + id] = b + j;
+              const bool keep = put && !(r2 > (bb ? keep_bb : keep_aa));
+              const unsigned entry = static_cast<unsigned>(j) | (bb ? 0x8000u : 0u);
+              if (KMAX == 1 || lk == 0) {
+                const unsigned kk = __ballot_sync(FULL, keep);
+                const int t = __shfl_sync(FULL, kept, g) + __popc(kk & lt);
+                if (keep && t < ROWS) S.ent[t * NT + id] = static_cast<unsigned short>(entry);
+                if (lane == g) kept += __popc(kk);
+              } else if (put && (q >> lk) < ROWS) {
+                // by its place in the bead's list, which says whose it is;
+                // the threads close the gaps afterwards
+                S.ent[(q >> lk) * NT + ((id << lk) | (q & kmask))] =
+                    static_cast<unsigned short>(keep ? entry : MD_NO_ENTRY);
+              }
+              if (lane == g) acc += __popc(mk);
+            }
+          }
+          if (mine_i >= 0) {
+            int full = acc;
+            if (full > a.max_nb) {
+              raise_error(a.err, ERR_NEIGHBOR_OVF, static_cast<uint32_t>(b + mine_i),
+                          static_cast<uint32_t>(full));
+              full = a.max_nb;
+            }
+            a.ncount[b + mine_i] = full;
+            S.n_ent[mine_i] = static_cast<unsigned short>(KMAX == 1 || lk == 0 ? kept : full);
+          }
+        }
+      }
+      __syncthreads();
+      n_ent = mine ? S.n_ent[i] : 0;
+      if (KMAX > 1 && lk > 0) {  // this thread's share of the bead's list, gaps closed
+        const int rows = mine ? (n_ent - sub + kmask) >> lk : 0;
+        n_ent = rows > ROWS ? rows : 0;
+        for (int t = 0; t < rows && rows <= ROWS; ++t) {
+          const unsigned short e = S.ent[t * NT + tid];
+          if (e != MD_NO_ENTRY) S.ent[n_ent++ * NT + tid] = e;
+        }
+      }
+      fits = !__syncthreads_or(n_ent > ROWS);
+    } else if (n_ent < 0) {  // the lists of an earlier launch
+      n_ent = 0;
+      if (mine) {
+        const int cnt = a.ncount[b + i];
+        const int* nl = a.nlist + b + i;
+        const size_t stride = static_cast<size_t>(a.n_mono_total);
+        const bool ai = S.amphi[i] != 0;
+        constexpr int PF = 4;
+        for (int q0 = sub; q0 < cnt; q0 += PF << lk) {
+          int js[PF];
+#pragma unroll
+          for (int u = 0; u < PF; ++u) {
+            const int q = q0 + (u << lk);
+            js[u] = q < cnt ? nl[static_cast<size_t>(q) * stride] - b : -1;
+          }
+#pragma unroll
+          for (int u = 0; u < PF; ++u) {
+            const int j = js[u];
+            if (j < 0) continue;
+            const float4 y = S.ref[j];
+            const float d0 = y.x - xv[0], d1 = y.y - xv[1], d2 = y.z - xv[2];
+            const bool bb = ai && S.amphi[j] != 0;
+            if (!((d0 * d0 + d1 * d1) + d2 * d2 > (bb ? keep_bb : keep_aa))) {
+              if (n_ent < ROWS)
+                S.ent[n_ent * NT + tid] = static_cast<unsigned short>(j | (bb ? 0x8000 : 0));
+              ++n_ent;
+            }
+          }
+        }
+      }
+      fits = !__syncthreads_or(n_ent > ROWS);
+    }
+    const bool want_epot = a.calc_epot && (step == total_steps - 1);
+    // forces (Box.cpp:243-286)
+    float F0 = 0.0f, F1 = 0.0f, F2 = 0.0f;
+    if (fits) {
+      // every bond end by a thread of its own, for the lead lanes below
+      for (int e = tid; e < n_bond; e += NT) {
+        const unsigned bd = S.bond[e];
+        const int j = static_cast<int>(bd & 0x7FFFu), ib = S.bead[e];
+        const float4 xb = pos[ib];
+        const float xx[3] = {xb.x, xb.y, xb.z};
+        float d[3], r2;
+        const bool anch = (bd & 0x8000u) != 0;
+        const float fa = md_bond_f32(a, pot, anch, pos[j], xx, d, &r2, b + ib, b + j);
+        if (want_epot) epot += md_fene_epot<float>(anch, r2);
+        S.bf[e] = make_float4(d[0], d[1], d[2], fa);
+      }
+      // Pairs, four at a time: their loads and arithmetic overlap (out of range
+      // the force is zero), the sums stay in list order.
+      for (int t0 = 0; t0 < n_ent; t0 += 4) {
+        float d0[4], d1[4], d2[4], fa[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int t = t0 + u < n_ent ? t0 + u : t0;
+          const unsigned e = S.ent[t * NT + tid];
+          const float4 y = pos[e & 0x7FFFu];
+          d0[u] = y.x - x[0];
+          d1[u] = y.y - x[1];
+          d2[u] = y.z - x[2];
+          const float r2 = (d0[u] * d0[u] + d1[u] * d1[u]) + d2[u] * d2[u];
+          fa[u] = pair_force_all(pot, (e & 0x8000u) != 0, r2, lambda, t0 + u < n_ent);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          F0 -= d0[u] * fa[u];
+          F1 -= d1[u] * fa[u];
+          F2 -= d2[u] * fa[u];
+        }
+      }
+      if (want_epot)
+        for (int t = 0; t < n_ent; ++t) {
+          const unsigned e = S.ent[t * NT + tid];
+          const float4 y = pos[e & 0x7FFFu];
+          const float d0 = y.x - x[0], d1 = y.y - x[1], d2 = y.z - x[2];
+          epot += md_pair_epot<float>(pot, (e & 0x8000u) != 0, (d0 * d0 + d1 * d1) + d2 * d2, lambda);
+        }
+      __syncthreads();  // the bonds are computed
+      if (mine && lead) {  // then added, in order
+        const int e1 = S.bstart[i + 1];
+        for (int e = S.bstart[i]; e < e1; ++e) {
+          const float4 g = S.bf[e];
+          F0 -= g.x * g.w;
+          F1 -= g.y * g.w;
+          F2 -= g.z * g.w;
+        }
+      }
+    } else if (mine) {
+      float F[3];
+      double ep = 0.0;
+      md_bead_forces_global(a, b, i, sub, lk, pos, S.amphi, pot, lambda, want_epot, F, &ep);
+      F0 = F[0]; F1 = F[1]; F2 = F[2];
+      epot += ep;
+    }
+    // partial forces of a bead's lanes (every lane of the warp takes part)
+    for (int o = 1; KMAX > 1 && o < (1 << lk); o <<= 1) {
+      F0 += __shfl_xor_sync(FULL, F0, o);
+      F1 += __shfl_xor_sync(FULL, F1, o);
+      F2 += __shfl_xor_sync(FULL, F2, o);
+    }
+    if (mine) {
+      f[0] = F0; f[1] = F1; f[2] = F2;
+      increment();
+      if (a.n_steps > 0) {
+        for (int d = 0; d < 3; ++d) v[d] += fk[d];  // second half kick
+        if (a.andersen) {  // (through a copy: the call would put v itself into memory)
+          float w[3] = {v[0], v[1], v[2]};
+          md_andersen_reset<float>(a, ri, r, step, i, md_step0, m, w);
+          for (int d = 0; d < 3; ++d) v[d] = w[d];
+        }
+      }
+    }
+  }
+  // write back
+  if (mine && lead) {
+    R4<float> p = ld4_rw(mpos, b + i);
+    p.x = x[0]; p.y = x[1]; p.z = x[2];
+    st4(mpos, b + i, p);
+    R4<float> vv = ld4_rw(mvel, b + i);
+    vv.x = v[0]; vv.y = v[1]; vv.z = v[2];
+    st4(mvel, b + i, vv);
+    st4(mfrc, b + i, R4<float>{f[0], f[1], f[2], 0.0f});
+    st4(mver, b + i, R4<float>{xv[0], xv[1], xv[2], 0.0f});
+  }
+  if (a.calc_epot) {
+    for (int o = 16; o > 0; o >>= 1) epot += __shfl_down_sync(FULL, epot, o);
+    if (lane == 0) s_red[tid >> 5] = epot;
+    __syncthreads();
+    if (tid == 0) {
+      double s = 0.0;
+      for (int w = 0; w < NT / 32; ++w) s += s_red[w];
+      a.dyn[r].epot = s;
+    }
+  }
+  if (tid == 0) {
+    a.dyn[r].verlet_rebuilds += rebuilds;
+    if (a.n_steps > 0) a.dyn[r].md_step = md_step0 + static_cast<unsigned long long>(a.n_steps);
+  }
+}
 
 // ---------------------------------------------------------------------------
 // The same substeps for one replica on a thread-block cluster of CS CTAs (CS

@@ -701,8 +701,14 @@ int upload_bonds(smpc_ctx* ctx) {
   // directed bond's source: the core owns its bonds, Molecule.cpp:146)
   const size_t M = static_cast<size_t>(ctx->total_mono);
   std::vector<std::vector<int2>> adj(M);
+  int* const max_ends = ctx->md_split.max_bond_ends;
+  max_ends[0] = max_ends[1] = 0;
   for (int r = 0; r < ctx->n_rep; ++r) {
     const int b = ctx->reps[r].mono_base;
+    if (!(ctx->reps[r].flags & smpc::REP_PERIODIC_MD)) {
+      int& m = max_ends[ctx->reps[r].n_mono > 512];
+      m = std::max(m, 2 * static_cast<int>(ctx->bsrc[r].size()));
+    }
     for (size_t k = 0; k < ctx->bsrc[r].size(); ++k) {
       const int s = ctx->bsrc[r][k], d = ctx->bdst[r][k];
       const int anch = ctx->anchor[r].empty() ? 0 : ctx->anchor[r][s];
