@@ -390,20 +390,19 @@ int md_cluster_size<Real>() {
 }
 
 #if SMPC_FAST_F32
-// list rows per thread: what fits beside the rest of MdFastSmem in an SM's
-// shared memory (1024 threads) or in half of it (512)
-constexpr int md_fast_rows(int nt) { return nt == 1024 ? 52 : 44; }
-template <int NT, int KMAX>
+// ROWS, list entries per thread: what fits beside the rest of MdFastSmem in an
+// SM's shared memory, or (512 threads with lanes per bead) in half of it. U: 2
+// to 4 pairs in flight measure the same, 1 and 8 are 10 % slower.
+template <int NT, int KMAX, int ROWS, int U = 4>
 static void md_fast(const MdArgs& a, int blocks, float* mpos, float* mvel, float* mfrc, float* mver,
                     cudaStream_t st) {
-  constexpr int ROWS = md_fast_rows(NT);
   constexpr size_t bytes = sizeof(MdFastSmem<NT, ROWS>);
-  static_assert(bytes + 1024 <= (NT == 1024 ? 227 : 113) * 1024, "shared memory");
-  static const bool set = cudaFuncSetAttribute(k_md_fast<NT, KMAX, ROWS>,
+  static_assert(bytes + 1024 <= (NT == 512 && KMAX > 1 ? 113 : 227) * 1024, "shared memory");
+  static const bool set = cudaFuncSetAttribute(k_md_fast<NT, KMAX, ROWS, U>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(bytes)) == cudaSuccess;
   (void)set;
-  k_md_fast<NT, KMAX, ROWS><<<blocks, NT, bytes, st>>>(a, mpos, mvel, mfrc, mver);
+  k_md_fast<NT, KMAX, ROWS, U><<<blocks, NT, bytes, st>>>(a, mpos, mvel, mfrc, mver);
 }
 #endif
 
@@ -424,8 +423,8 @@ void launch_md<Real>(const MdArgs& a, int n_rep, Real* mpos, Real* mvel, Real* m
   MdArgs b = a;
 #if SMPC_FAST_F32
   // Lists in shared memory wherever the thermostat and the number of bonds allow
-  // it: 256 stars of 121 to 721 beads take 207 us instead of 337 per cycle of
-  // 10 substeps, one of 401 beads 69 us instead of 128.
+  // it: 256 stars of 121 to 721 beads take 135 us instead of 337 per cycle of
+  // 10 substeps, one of 121 beads 35 us instead of 128.
   const int* const ends = split.max_bond_ends;
   const bool fast = !a.lowe && std::max(ends[0], ends[1]) <= md_fast_bonds(1024);
   if (variant == 3 && split.n_big > 0 && split.n_big < n_rep && a.order) {
@@ -433,13 +432,13 @@ void launch_md<Real>(const MdArgs& a, int n_rep, Real* mpos, Real* mvel, Real* m
     cudaEventRecord(split.fork, st);
     cudaStreamWaitEvent(split.st2, split.fork, 0);
     if (fast)
-      md_fast<1024, 8>(b, split.n_big, mpos, mvel, mfrc, mver, split.st2);
+      md_fast<1024, 8, 60>(b, split.n_big, mpos, mvel, mfrc, mver, split.st2);
     else
       k_md_substeps<Real, 1024, 1, 8><<<split.n_big, 1024, 0, split.st2>>>(b, mpos, mvel, mfrc, mver);
     MdArgs c = a;
     c.order = a.order + split.n_big;
     if (fast && ends[0] <= md_fast_bonds(512))
-      md_fast<512, 8>(c, n_rep - split.n_big, mpos, mvel, mfrc, mver, st);
+      md_fast<512, 8, 52>(c, n_rep - split.n_big, mpos, mvel, mfrc, mver, st);
     else
       k_md_substeps<Real, 512, 1, 8><<<n_rep - split.n_big, 512, 0, st>>>(c, mpos, mvel, mfrc, mver);
     cudaEventRecord(split.join, split.st2);
@@ -448,7 +447,7 @@ void launch_md<Real>(const MdArgs& a, int n_rep, Real* mpos, Real* mvel, Real* m
   }
   if (variant == 2 || variant == 3) {
     if (fast)
-      md_fast<1024, 8>(b, n_rep, mpos, mvel, mfrc, mver, st);
+      md_fast<1024, 8, 60>(b, n_rep, mpos, mvel, mfrc, mver, st);
     else
       k_md_substeps<Real, 1024, 1, 8><<<n_rep, 1024, 0, st>>>(b, mpos, mvel, mfrc, mver);
     return;
@@ -459,7 +458,12 @@ void launch_md<Real>(const MdArgs& a, int n_rep, Real* mpos, Real* mvel, Real* m
     return;
   }
   if (fast) {
-    md_fast<1024, 1>(b, n_rep, mpos, mvel, mfrc, mver, st);
+    // Up to 512 beads everywhere: half the threads, with twice the registers
+    // (no spills): one star of 121 beads 35 us per cycle against 39 with 1,024.
+    if (split.n_big == 0 && ends[0] <= md_fast_bonds(512))
+      md_fast<512, 1, 128>(b, n_rep, mpos, mvel, mfrc, mver, st);
+    else
+      md_fast<1024, 1, 60>(b, n_rep, mpos, mvel, mfrc, mver, st);
     return;
   }
 #endif

@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 #include <stdint.h>
 
+#include "exact_div.cuh"
 #include "mpc_kernels.cuh"
 #include "smpc_device.cuh"
 
@@ -70,12 +71,12 @@ __device__ __forceinline__ R pair_force(int pot, bool bb, R r2, R lambda) {
 }
 
 // FP32: 1/r2 as the correctly rounded reciprocal (the same bits as the
-// division, without its general path)
+// division, without its general path, which took half of the pair loop)
 template <>
 __device__ __forceinline__ float pair_force<float>(int pot, bool bb, float r2, float lambda) {
   if (pot == POT_REF4824) {
     if (r2 < 1.0594631f || (bb && r2 < 2.25f)) {
-      const float rm2 = __frcp_rn(r2);
+      const float rm2 = rcp_exact(r2);
       float rm24 = rm2 * rm2 * rm2;
       rm24 *= rm24;
       rm24 *= rm24;
@@ -85,7 +86,7 @@ __device__ __forceinline__ float pair_force<float>(int pot, bool bb, float r2, f
     return 0.0f;
   }
   if (r2 < 1.2599210498948732f || (bb && r2 < 6.25f)) {
-    const float rm2 = __frcp_rn(r2);
+    const float rm2 = rcp_exact(r2);
     const float rm6 = rm2 * rm2 * rm2;
     const float f = 48.0f * rm2 * rm6 * (rm6 - 0.5f);
     return r2 < 1.2599210498948732f ? f : lambda * f;
@@ -93,22 +94,27 @@ __device__ __forceinline__ float pair_force<float>(int pot, bool bb, float r2, f
   return 0.0f;
 }
 
-// pair_force<float> without a branch around the arithmetic (zero out of range
-// and where `use` is false)
-__device__ __forceinline__ float pair_force_all(int pot, bool bb, float r2, float lambda, bool use) {
-  if (pot == POT_REF4824) {
-    const bool core = r2 < 1.0594631f, in = use && (core || (bb && r2 < 2.25f));
-    const float rm2 = __frcp_rn(in ? r2 : 1.0f);
+// pair_force<float> without branches, so that several pairs overlap: zero out of
+// range and where `use` is false; special is set where r2 wants the general
+// reciprocal (the caller then takes pair_force).
+__device__ __forceinline__ float pair_force_all(int pot, bool bb, float r2, float lambda, bool use,
+                                                bool& special) {
+  const bool ref = pot == POT_REF4824;
+  const bool core = r2 < (ref ? 1.0594631f : 1.2599210498948732f);
+  const bool in = use && (core || (bb && r2 < (ref ? 2.25f : 6.25f)));
+  const float s2 = in ? r2 : 1.0f;
+  special = special || !rcp_has_range(s2);
+  const float rm2 = rcp_in_range(s2);
+  float f;
+  if (ref) {
     float rm24 = rm2 * rm2 * rm2;
     rm24 *= rm24;
     rm24 *= rm24;
-    const float f = 192.0f * rm2 * rm24 * (rm24 - 0.5f);
-    return in ? (core ? f : lambda * f) : 0.0f;
+    f = 192.0f * rm2 * rm24 * (rm24 - 0.5f);
+  } else {
+    const float rm6 = rm2 * rm2 * rm2;
+    f = 48.0f * rm2 * rm6 * (rm6 - 0.5f);
   }
-  const bool core = r2 < 1.2599210498948732f, in = use && (core || (bb && r2 < 6.25f));
-  const float rm2 = __frcp_rn(in ? r2 : 1.0f);
-  const float rm6 = rm2 * rm2 * rm2;
-  const float f = 48.0f * rm2 * rm6 * (rm6 - 0.5f);
   return in ? (core ? f : lambda * f) : 0.0f;
 }
 
@@ -177,7 +183,7 @@ __device__ __forceinline__ R fene_force(bool anchor, R r2) {
 }
 template <>
 __device__ __forceinline__ float fene_force<float>(bool anchor, float r2) {
-  return -30.0f * __frcp_rn(1.0f - r2 * (anchor ? 1.0f / 20.25f : 1.0f / 2.25f));
+  return -30.0f * rcp_exact(1.0f - r2 * (anchor ? 1.0f / 20.25f : 1.0f / 2.25f));
 }
 template <typename R>
 __device__ __forceinline__ R fene_pot(bool anchor, R r2) {
@@ -412,8 +418,10 @@ __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, 
   static_assert(MD_BUCKETS == 2048, "11-bit bucket field");
   static_assert(MD_BUCKETS % NT == 0 && NT % 32 == 0, "bucket scan layout");
   constexpr int PER = MD_BUCKETS / NT;
+#pragma unroll 1
   for (int t = threadIdx.x; t <= MD_BUCKETS; t += NT) s_start[t] = 0;
   __syncthreads();
+#pragma unroll 1
   for (int j = threadIdx.x; j < n; j += NT) {
     const int bk = s_bkt[j];
     s_bkt[j] = bk | (atomicAdd(s_start + bk, 1) << 11);
@@ -428,6 +436,7 @@ __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, 
     if ((threadIdx.x & 31u) == 31u) s_wsum[threadIdx.x >> 5] = inc;
     __syncthreads();
     int wbase = 0;
+#pragma unroll 1
     for (int w = 0; w < static_cast<int>(threadIdx.x >> 5); ++w) wbase += s_wsum[w];
     int run = wbase + inc - tot;
 #pragma unroll
@@ -435,16 +444,20 @@ __device__ __forceinline__ void md_bucket_sort(int n, int* s_bkt, int* s_start, 
     if (threadIdx.x == NT - 1) s_start[MD_BUCKETS] = run;
   }
   __syncthreads();
+#pragma unroll 1
   for (int j = threadIdx.x; j < n; j += NT)
     s_sorted[s_start[s_bkt[j] & 2047] + (s_bkt[j] >> 11)] = j;
   __syncthreads();
+#pragma unroll 1
   for (int j = threadIdx.x; j < n; j += NT) {
     const int bk = s_bkt[j] & 2047;
     int place = 0;
+#pragma unroll 1
     for (int k = s_start[bk]; k < s_start[bk + 1]; ++k) place += s_sorted[k] < j ? 1 : 0;
     s_bkt[j] = bk | (place << 11);
   }
   __syncthreads();
+#pragma unroll 1
   for (int j = threadIdx.x; j < n; j += NT)
     s_sorted[s_start[s_bkt[j] & 2047] + (s_bkt[j] >> 11)] = j;
   __syncthreads();
@@ -845,39 +858,50 @@ __device__ __noinline__ void md_bead_forces_lists(const MdArgs& a, int b, int i,
 //    beads that do not attract act on each other up to 1.12 only, and their
 //    pairs beyond 1.12 + skin carry exactly zero force until then. About a
 //    third of the entries are left, and none is read from L2 in a substep.
-//  * Rebuilds: a warp takes one occupied cell at a time. All beads of a cell
-//    have the same 27 neighbour cells, so the warp lists those cells' members
-//    once, 32 candidates at a time, and tests them against every bead of the
-//    cell; ballots keep the order (cells, then beads, ascending) in which one
-//    lane walking alone would find them. That walk took 78,000 cycles for 121
-//    beads and 97,000 for 401, seven tenths of the kernel's time at the one
-//    rebuild in five substeps of a relaxed star; this takes 14,000 and 39,000.
+//  * Rebuilds (md_fast_build) sort the beads instead of walking 27 hash cells
+//    per bead, which took 78,000 cycles for 121 beads and 97,000 for 401, seven
+//    tenths of the kernel's time at the one rebuild in five substeps of a
+//    relaxed star; they take 10,000 and 31,000.
 //  * Bonds are in shared memory; every bond end is computed by a thread of its
 //    own and added in order by its bead's lead lane (a star's core has one
 //    bond per arm).
 //  * The half-kick increment is computed once per force evaluation, and
 //    positions alternate between two buffers: two barriers per substep.
+//  * A CTA's time is latencies and its warps' own instruction counts: few warps,
+//    one dependent phase after another. So what most substeps do not do is out
+//    of line (its code and registers cost 10 to 15 %), and the pairs' reciprocals
+//    carry no branch (half of the pair loop).
+// 10 substeps of 256 stars of 121 to 721 beads take 135 us instead of 337, of
+// 32 of them 126 instead of 316, of one of 121 beads 35 instead of 128.
 constexpr unsigned short MD_NO_ENTRY = 0xFFFFu;
 // Bond ends of a replica (two per bond) that fit: a star of NT beads has NT - 1 bonds.
 constexpr int md_fast_bonds(int nt) { return 2 * nt; }
 template <int NT, int ROWS>
 struct MdFastSmem {
   static constexpr int BONDS = md_fast_bonds(NT);
+  // entry t of thread T at t ST + T: partner | attracting << 15; consecutive
+  // entries of a thread lie in different banks
+  static constexpr int ST = NT + 2;
   float4 pos[2][NT];              // positions, by substep parity
   float4 ref[NT];                 // positions at the last list build
-  float4 bf[BONDS];               // per bond end: the bond's vector and force factor
-  int head[MD_BUCKETS + 1];       // bucket starts in sorted
-  int sorted[NT];                 // beads by bucket
-  int bucket[NT];                 // bucket of each bead
-  int ckey[NT];                   // cell of each bead
-  unsigned short ent[ROWS * NT];  // entry t of thread T at t NT + T: partner | attracting << 15
-  unsigned short n_ent[NT];
-  unsigned short cells[NT];       // place in sorted of every occupied cell's first bead
+  union {
+    float4 bf[BONDS];             // per bond end: the bond's vector and force factor
+    struct {                      // during a list build
+      // by sorted order, a gap after every eight against bank conflicts:
+      // position, largest squared distance kept
+      float4 spos[NT + NT / 8];
+      unsigned key[NT];           // (cell z, y, x, bead); then 128 octets in reach per warp
+      float box[6][NT / 8];       // of every octet by sorted order: lower, upper corner
+    };
+  };
+  int sorted[NT];                 // beads by (cell, bead): bead | attracting << 15
+  unsigned short ent[ROWS * ST];
+  unsigned short n_ent[NT];       // entries of each thread
   unsigned short bond[BONDS];     // per bond end: partner | anchor bond << 15
   unsigned short bead[BONDS];     // and the bead itself
   unsigned short bstart[NT + 2];
   unsigned char amphi[NT];
-  int n_cells, next_cell;
+  int next_group;
   float core_ref[3];
 };
 // Squared distance at the list build up to which a pair is kept: its cut-off
@@ -888,6 +912,10 @@ __device__ __forceinline__ float md_keep_r2(int pot, bool bb, float skin) {
                                         : (bb ? 6.25f : 1.2599210498948732f);
   const float r = sqrtf(cut2) + fmaxf(skin, 0.0f) + 1e-3f;
   return r * r;
+}
+
+static __device__ __noinline__ void md_fene_error(ErrorState* err, uint32_t i, uint32_t j) {
+  raise_error(err, ERR_FENE, i, j);
 }
 
 // FENE bond of a bead at x with one at y: its vector d and force factor.
@@ -901,7 +929,7 @@ __device__ __forceinline__ float md_bond_f32(const MdArgs& a, int pot, bool anch
   if (pot == POT_REF4824) {
     // reference FENE: beyond R0 the force changes sign (Potentials.h:24-55)
     if (r2 >= (anch ? 20.25f : 2.25f))
-      raise_error(a.err, ERR_FENE, static_cast<uint32_t>(gi), static_cast<uint32_t>(gj));
+      md_fene_error(a.err, static_cast<uint32_t>(gi), static_cast<uint32_t>(gj));
   } else {
     // 12-6 preset: FENE argument capped at 0.98 R0^2 (finite, restoring)
     const float cap = (anch ? 20.25f : 2.25f) * 0.98f;
@@ -953,8 +981,322 @@ static __device__ __noinline__ void md_bead_forces_global(const MdArgs& a, int b
   F[2] = F2;
 }
 
+// Verlet lists: every other bead within r_verlet (Box.cpp:146-179), ordered by
+// (cell, bead) over the 27 cells of side r_verlet around the bead's own.
+// Returns the number of this thread's entries. Sorting the beads by cell (z,
+// then y, then x) and bead puts every list into that order, so that no cell
+// has to be looked up: a warp takes an octet of beads in that order, four lanes
+// each, and tests them against the octets whose boxes are in reach, an octet
+// per lane. Of the 31,000 cycles for 401 beads the tests take a quarter, the
+// entries half.
 template <int NT, int KMAX, int ROWS>
-__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1)
+static __device__ __noinline__ int md_fast_build(int* nlist, int* ncount, int n_mono_total,
+                                                 int max_nb, ErrorState* err, int b, int n, int lk,
+                                                 int buf, float rv, float keep_bb, float keep_aa) {
+  constexpr unsigned FULL = 0xFFFFFFFFu;
+  typedef MdFastSmem<NT, ROWS> Smem;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  Smem& S = *reinterpret_cast<Smem*>(s_dyn);
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
+  const int warps = (n + 31) >> 5;
+  // Each warp sorts its 32 beads' keys; a key's place among all is its place
+  // there plus, for every other warp, the number of smaller keys. (A bitonic
+  // sort of all took four times as long: 55 dependent steps for 721 beads.)
+  // Cells count from bead 0's, within 64 of it on either side; what lies
+  // further out is listed all the same, in another order.
+  unsigned key = ~0u;
+  if (tid < 32 * warps) {
+    if (tid < n) {
+      const float4 p = S.pos[buf][tid], o = S.pos[buf][0];
+      const float inv_rv = 1.0f / rv;
+      const float c[3] = {p.z, p.y, p.x}, c0[3] = {o.z, o.y, o.x};
+      key = 0u;
+      for (int d = 0; d < 3; ++d) {
+        const float k = floorf(c[d] * inv_rv) - floorf(c0[d] * inv_rv);
+        key = key << 7 | static_cast<unsigned>(static_cast<int>(fminf(fmaxf(k, -64.0f), 63.0f)) + 64);
+      }
+      key = key << 10 | static_cast<unsigned>(tid);
+      S.ref[tid] = p;
+      if (tid == 0) {
+        S.core_ref[0] = p.x; S.core_ref[1] = p.y; S.core_ref[2] = p.z;
+        S.next_group = 0;
+      }
+    }
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+      for (int stride = size >> 1; stride > 0; stride >>= 1) {
+        const unsigned other = __shfl_xor_sync(FULL, key, stride);
+        const bool low = ((lane & stride) == 0) == (size == 32 || (lane & size) == 0);
+        key = low ? min(key, other) : max(key, other);
+      }
+    S.key[tid] = key;
+  }
+  __syncthreads();
+  if (tid < 32 * warps) {
+    int rank = lane;
+#pragma unroll 2
+    for (int w = 0; w < warps; ++w) {
+      const unsigned* run = S.key + 32 * w;
+      int at = 0;
+#pragma unroll
+      for (int st = 16; st > 0; st >>= 1) at += run[at + st - 1] < key ? st : 0;
+      at += run[at] < key ? 1 : 0;
+      rank += w == tid >> 5 ? 0 : at;
+    }
+    if (key != ~0u) {
+      const int id = static_cast<int>(key & 1023u);
+      const int bb = S.amphi[id] != 0 ? 0x8000 : 0;
+      float4 p = S.pos[buf][id];
+      p.w = bb ? keep_bb : keep_aa;
+      S.spos[rank + (rank >> 3)] = p;
+      S.sorted[rank] = id | bb;
+    }
+    if (tid >= n) S.spos[tid + (tid >> 3)] = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+  }
+  __syncthreads();
+  if (tid < 32 * warps) {  // the octets' boxes, of their beads only
+    const float4 p = S.spos[tid + (tid >> 3)];
+    float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
+    if (tid >= n) hi[0] = hi[1] = hi[2] = -INFINITY;
+#pragma unroll 1
+    for (int o = 4; o > 0; o >>= 1)
+      for (int d = 0; d < 3; ++d) {
+        lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
+        hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
+      }
+    if ((lane & 7) == 0)
+      for (int d = 0; d < 3; ++d) {
+        S.box[d][tid >> 3] = lo[d];
+        S.box[3 + d][tid >> 3] = hi[d];
+      }
+  }
+  __syncthreads();
+  const float rv2 = rv * rv;
+  const int octets = (n + 7) >> 3, kmask = (1 << lk) - 1;
+  const int part = lane & 3;
+  unsigned char* const near = reinterpret_cast<unsigned char*>(S.key) + 128 * (tid >> 5);
+#pragma unroll 1
+  for (;;) {
+    int g = 0;
+    if (lane == 0) g = atomicAdd(&S.next_group, 1);
+    g = __shfl_sync(FULL, g, 0);
+    if (g >= octets) break;
+    // the octets in reach: the distance of the boxes, rounded like the beads' own
+    int n_near = 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < octets; c0 += 32) {
+      const int c = min(c0 + lane, octets - 1);
+      float q[3];
+      for (int d = 0; d < 3; ++d)
+        q[d] = fmaxf(fmaxf(S.box[d][c] - S.box[3 + d][g], S.box[d][g] - S.box[3 + d][c]), 0.0f);
+      const float r2 = __fmaf_rn(q[2], q[2], __fmaf_rn(q[0], q[0], __fmul_rn(q[1], q[1])));
+      const bool reach = c0 + lane < octets && r2 <= rv2;
+      const unsigned mk = __ballot_sync(FULL, reach);
+      if (reach) near[n_near + __popc(mk & ((1u << lane) - 1u))] = static_cast<unsigned char>(c);
+      n_near += __popc(mk);
+    }
+    __syncwarp();
+    const int s = 8 * g + (lane >> 2);
+    const bool real = s < n;
+    const float4 xi = S.spos[s + (s >> 3)];
+    const int me = S.sorted[s], id = me & 0x7FFF;
+    int acc = 0, kept = 0;  // the bead's list entries so far, and those of them that are kept
+#pragma unroll 1
+    for (int c0 = 0; c0 < n_near; c0 += 4) {  // an octet for each of the bead's lanes
+      unsigned in = 0u, keep = 0u;
+      const int c = near[min(c0 + part, n_near - 1)];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float4 y = S.spos[9 * c + k];
+        const float d0 = y.x - xi.x, d1 = y.y - xi.y, d2 = y.z - xi.z;
+        const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d0, d0, __fmul_rn(d1, d1)));
+        if (r2 <= rv2) in |= 1u << k;
+        if (r2 <= fminf(y.w, xi.w)) keep |= 1u << k;  // keep_bb: both attract
+      }
+      if (c == g) in &= ~(1u << (lane >> 2));  // the bead itself
+      if (8 * c + 8 > n) in &= (1u << (n - 8 * c)) - 1u;  // (an infinite r_verlet)
+      if (!real || c0 + part >= n_near) in = 0u;
+      keep &= in;
+      unsigned all = in << (8 * part), all_keep = keep << (8 * part);  // of the bead's four lanes
+      all |= __shfl_xor_sync(FULL, all, 1);
+      all |= __shfl_xor_sync(FULL, all, 2);
+      all_keep |= __shfl_xor_sync(FULL, all_keep, 1);
+      all_keep |= __shfl_xor_sync(FULL, all_keep, 2);
+      // nothing past the list's capacity is kept
+      const int found = __popc(all);
+#pragma unroll 1
+      for (int drop = acc + found - max_nb; drop > 0 && all != 0u; --drop)
+        all ^= 0x80000000u >> __clz(all);
+      all_keep &= all;
+      // its entries in turn to its lanes, so that a full octet is not one lane's work
+      unsigned rest = all;
+      int q = acc + part;
+      for (int p = 0; p < part; ++p) rest &= rest - 1u;
+#pragma unroll 1
+      while (rest != 0u) {
+        const int k = __ffs(rest) - 1;
+        const unsigned bit = 1u << k;
+        const int other = S.sorted[8 * near[c0 + (k >> 3)] + (k & 7)], j = other & 0x7FFF;
+        nlist[static_cast<size_t>(q) * n_mono_total + id] = b + j;
+        const unsigned short entry = static_cast<unsigned short>(j | (other & me & 0x8000));
+        const bool kp = (all_keep & bit) != 0u;
+        if (KMAX == 1 || lk == 0) {
+          const int t = kept + __popc(all_keep & (bit - 1u));
+          if (kp && t < ROWS) S.ent[t * Smem::ST + id] = entry;
+        } else if ((q >> lk) < ROWS) {
+          // by its place in the list, which says whose it is; the threads close
+          // the gaps afterwards
+          S.ent[(q >> lk) * Smem::ST + ((id << lk) | (q & kmask))] = kp ? entry : MD_NO_ENTRY;
+        }
+        q += 4;
+        for (int p = 0; p < 4; ++p) rest &= rest - 1u;
+      }
+      acc += found;
+      kept += __popc(all_keep);
+    }
+    __syncwarp();  // near is read
+    if (real && part == 0) {
+      if (acc > max_nb) {
+        raise_error(err, ERR_NEIGHBOR_OVF, static_cast<uint32_t>(b + id),
+                    static_cast<uint32_t>(acc));
+        acc = max_nb;
+      }
+      ncount[id] = acc;
+      S.n_ent[id] = static_cast<unsigned short>(KMAX == 1 || lk == 0 ? kept : acc);
+    }
+  }
+  __syncthreads();
+  const int i = tid >> lk, sub = tid & kmask;
+  int n_ent = i < n ? S.n_ent[i] : 0;
+  if (KMAX > 1 && lk > 0) {  // this thread's share of the bead's list, gaps closed
+    const int rows = i < n ? (n_ent - sub + kmask) >> lk : 0;
+    n_ent = rows > ROWS ? rows : 0;
+#pragma unroll 1
+    for (int t = 0; t < rows && rows <= ROWS; ++t) {
+      const unsigned short e = S.ent[t * Smem::ST + tid];
+      if (e != MD_NO_ENTRY) S.ent[n_ent++ * Smem::ST + tid] = e;
+    }
+  }
+  return n_ent;
+}
+
+// The same from the lists of an earlier launch.
+template <int NT, int KMAX, int ROWS>
+static __device__ __noinline__ int md_fast_take(const int* nlist, const int* ncount, int n_mono_total,
+                                                int b, int n, int lk, float keep_bb,
+                                                float keep_aa) {
+  typedef MdFastSmem<NT, ROWS> Smem;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  Smem& S = *reinterpret_cast<Smem*>(s_dyn);
+  const int tid = static_cast<int>(threadIdx.x), lane = tid & 31;
+  // Lanes per bead here: those of the substep, or, where that is one, as many
+  // as there are threads for; entries are then appended in order by ballots.
+  int lt = lk;
+  while (lk == 0 && lt < 3 && (n << (lt + 1)) <= NT) ++lt;
+  const int i = tid >> lt, sub = tid & ((1 << lt) - 1);
+  const unsigned team = ((1u << (1 << lt)) - 1u) << (lane & ~((1 << lt) - 1));
+  const unsigned before = team & ((1u << lane) - 1u);
+  int n_ent = 0;
+  const int cnt = i < n ? ncount[i] : 0;
+  float4 xr = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  bool ai = false;
+  if (i < n) {
+    xr = S.ref[i];
+    ai = S.amphi[i] != 0;
+  }
+  const int* nl = nlist + i;
+  const size_t stride = static_cast<size_t>(n_mono_total);
+  constexpr int PF = 8;  // loads in flight
+#pragma unroll 1
+  for (int q0 = sub; __any_sync(0xFFFFFFFFu, q0 < cnt); q0 += PF << lt) {
+    int js[PF];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int q = q0 + (u << lt);
+      js[u] = q < cnt ? nl[static_cast<size_t>(q) * stride] - b : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int j = max(js[u], 0);
+      const float4 y = S.ref[j];
+      const float d0 = y.x - xr.x, d1 = y.y - xr.y, d2 = y.z - xr.z;
+      const bool bb = ai && S.amphi[j] != 0;
+      const bool keep =
+          js[u] >= 0 && !((d0 * d0 + d1 * d1) + d2 * d2 > (bb ? keep_bb : keep_aa));
+      const unsigned short entry = static_cast<unsigned short>(j | (bb ? 0x8000 : 0));
+      if (KMAX > 1 && lk > 0) {  // this thread's own
+        if (keep && n_ent < ROWS) S.ent[n_ent * Smem::ST + tid] = entry;
+        n_ent += keep ? 1 : 0;
+      } else {
+        const unsigned mk = __ballot_sync(0xFFFFFFFFu, keep);
+        const int t = n_ent + __popc(mk & before);
+        if (keep && t < ROWS) S.ent[t * Smem::ST + i] = entry;
+        n_ent += __popc(mk & team);
+      }
+    }
+  }
+  if (lt == lk) return n_ent;
+  if (sub == 0 && i < n) S.n_ent[i] = static_cast<unsigned short>(n_ent);
+  __syncthreads();
+  return tid < n ? S.n_ent[tid] : 0;
+}
+
+static __device__ __noinline__ float pair_force_general(int pot, bool bb, float r2, float lambda) {
+  return pair_force<float>(pot, bb, r2, lambda);
+}
+
+// One thread's share of a substep's forces: every bond end by a thread of its
+// own, for the lead lanes to add, and its list entries, U at a time (their
+// loads and arithmetic overlap, out of range the force is zero), summed in
+// list order.
+template <int NT, int ROWS, int POT, int U>
+__device__ __forceinline__ void md_fast_forces(MdFastSmem<NT, ROWS>& S, const MdArgs& a, int b,
+                                               const float4* pos, int n_bond, int n_ent,
+                                               const float* x, float lambda, float& F0, float& F1,
+                                               float& F2) {
+  const int tid = static_cast<int>(threadIdx.x);
+#pragma unroll 1
+  for (int e = tid; e < n_bond; e += NT) {
+    const unsigned bd = S.bond[e];
+    const int j = static_cast<int>(bd & 0x7FFFu), ib = S.bead[e];
+    const float4 xb = pos[ib];
+    const float xx[3] = {xb.x, xb.y, xb.z};
+    float d[3], r2;
+    const float fa = md_bond_f32(a, POT, (bd & 0x8000u) != 0, pos[j], xx, d, &r2, b + ib, b + j);
+    S.bf[e] = make_float4(d[0], d[1], d[2], fa);
+  }
+#pragma unroll 1
+  for (int t0 = 0; t0 < n_ent; t0 += U) {
+    float d0[U], d1[U], d2[U], fa[U];
+    bool special = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + u < n_ent ? t0 + u : t0;
+      const unsigned e = S.ent[t * S.ST + tid];
+      const float4 y = pos[e & 0x7FFFu];
+      d0[u] = y.x - x[0];
+      d1[u] = y.y - x[1];
+      d2[u] = y.z - x[2];
+      const float r2 = (d0[u] * d0[u] + d1[u] * d1[u]) + d2[u] * d2[u];
+      fa[u] = pair_force_all(POT, (e & 0x8000u) != 0, r2, lambda, t0 + u < n_ent, special);
+    }
+    if (special)  // beads in one place, or not a number
+      for (int u = 0; u < U; ++u)
+        if (t0 + u < n_ent)
+          fa[u] = pair_force_general(POT, (S.ent[(t0 + u) * S.ST + tid] & 0x8000u) != 0,
+                                     (d0[u] * d0[u] + d1[u] * d1[u]) + d2[u] * d2[u], lambda);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      F0 -= d0[u] * fa[u];
+      F1 -= d1[u] * fa[u];
+      F2 -= d2[u] * fa[u];
+    }
+  }
+}
+
+template <int NT, int KMAX, int ROWS, int U>
+__global__ void __launch_bounds__(NT, NT == 512 && KMAX > 1 ? 2 : 1)
     k_md_fast(MdArgs a, float* mpos, float* mvel, float* mfrc, float* mver) {
   static_assert(NT <= 1024, "list entries hold 10-bit partners");
   constexpr unsigned FULL = 0xFFFFFFFFu;
@@ -977,7 +1319,6 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1)
   const float dth = dt * 0.50f;
   const float lambda = static_cast<float>(ri.lambda);
   const float rv = static_cast<float>(ri.r_verlet);
-  const float rv2 = rv * rv;
   const float skin = rv - static_cast<float>(ri.r_cut);
   const float lim = skin * 0.5f;
   const int pot = ri.potential;
@@ -985,14 +1326,21 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1)
   const unsigned long long md_step0 = a.dyn[r].md_step;  // thread 0 adds n_steps at the end
 
   float x[3] = {0, 0, 0}, v[3] = {0, 0, 0}, f[3] = {0, 0, 0}, fk[3] = {0, 0, 0}, xv[3] = {0, 0, 0},
-        m = 1.0f;
-  auto increment = [&]() {  // f / m dt / 2 of the half kicks (Thermostat_None.cpp:22,34)
-    for (int d = 0; d < 3; ++d) fk[d] = a.andersen ? f[d] * (dth / m) : (f[d] / m) * dth;
+        m = 1.0f, rm = 1.0f, c_andersen = 0.0f;
+  // f / m dt / 2 of the half kicks (Thermostat_None.cpp:22,34)
+  auto increment = [&]() {
+    if (a.andersen) {
+      for (int d = 0; d < 3; ++d) fk[d] = f[d] * c_andersen;
+    } else {
+      for (int d = 0; d < 3; ++d) fk[d] = div_exact(f[d], m, rm) * dth;
+    }
   };
   if (mine) {
     const R4<float> p = ld4_rw(mpos, b + i), vv = ld4_rw(mvel, b + i), ff = ld4_rw(mfrc, b + i),
                     pv = ld4_rw(mver, b + i);
     x[0] = p.x; x[1] = p.y; x[2] = p.z; m = p.w;
+    rm = rcp_exact(m);
+    c_andersen = dth / m;
     v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
     f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
     xv[0] = pv.x; xv[1] = pv.y; xv[2] = pv.z;
@@ -1054,226 +1402,24 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1)
       }
     }
     if (__syncthreads_or(over)) {
-      // Verlet lists: every other bead within r_verlet (Box.cpp:146-179), found
-      // through a hashed grid of side r_verlet
       ++rebuilds;
-      const float inv_rv = 1.0f / rv;
-      for (int j = tid; j < n; j += NT) {
-        const float4 p = pos[j];
-        const int cx = static_cast<int>(floorf(p.x * inv_rv)),
-                  cy = static_cast<int>(floorf(p.y * inv_rv)),
-                  cz = static_cast<int>(floorf(p.z * inv_rv));
-        S.ckey[j] = md_cell_key(cx, cy, cz);
-        S.bucket[j] = md_bucket(cx, cy, cz);
-        S.ref[j] = p;
-      }
-      if (tid == 0) {
-        S.n_cells = S.next_cell = 0;
-        S.core_ref[0] = pos[0].x; S.core_ref[1] = pos[0].y; S.core_ref[2] = pos[0].z;
-      }
       xv[0] = x[0]; xv[1] = x[1]; xv[2] = x[2];
-      __syncthreads();
-      md_bucket_sort<NT>(n, S.bucket, S.head, S.sorted);
-      // the occupied cells, each by the place of its first bead
-      for (int p = tid; p < n; p += NT) {
-        const int key = S.ckey[S.sorted[p]];
-        const int bk = S.bucket[S.sorted[p]] & (MD_BUCKETS - 1);
-        bool first = true;
-        for (int q = S.head[bk]; q < p && first; ++q) first = S.ckey[S.sorted[q]] != key;
-        if (first) S.cells[atomicAdd(&S.n_cells, 1)] = static_cast<unsigned short>(p);
-      }
-      __syncthreads();
-      const unsigned lt = (1u << lane) - 1u;
-      for (;;) {
-        int cell = 0;
-        if (lane == 0) cell = atomicAdd(&S.next_cell, 1);
-        cell = __shfl_sync(FULL, cell, 0);
-        if (cell >= S.n_cells) break;
-        const int p0 = S.cells[cell];
-        const int j0 = S.sorted[p0], key0 = S.ckey[j0];
-        const float4 c = pos[j0];
-        const int cx = static_cast<int>(floorf(c.x * inv_rv)),
-                  cy = static_cast<int>(floorf(c.y * inv_rv)),
-                  cz = static_cast<int>(floorf(c.z * inv_rv));
-        // lanes 0..26: one neighbour cell each
-        int want = 0, start = 0, cnt = 0;
-        if (lane < 27) {
-          const int tx = cx + lane % 3 - 1, ty = cy + (lane / 3) % 3 - 1, tz = cz + lane / 9 - 1;
-          want = md_cell_key(tx, ty, tz);
-          const int bk = md_bucket(tx, ty, tz);
-          start = S.head[bk];
-          cnt = S.head[bk + 1] - start;
-        }
-        const int incl = md_warp_scan(cnt);
-        const int excl = incl - cnt;
-        const int total = __shfl_sync(FULL, incl, 31);
-        const int pend = S.head[md_bucket(cx, cy, cz) + 1];
-        for (int pb = p0; pb < pend;) {
-          // up to 32 beads of the cell: lane g holds the g-th and its counts
-          int mine_i = -1, acc = 0, kept = 0, n_b = 0, pn = pb;
-          for (; pn < pend && n_b < 32; pn += 32) {
-            const int jj = pn + lane < pend ? S.sorted[pn + lane] : -1;
-            unsigned mk = __ballot_sync(FULL, jj >= 0 && S.ckey[jj < 0 ? 0 : jj] == key0);
-            if (n_b + __popc(mk) > 32) break;  // the rest in another pass over the candidates
-            while (mk) {
-              const int src = __ffs(mk) - 1;
-              const int id = __shfl_sync(FULL, jj, src);
-              if (lane == n_b) mine_i = id;
-              ++n_b;
-              mk &= mk - 1;
-            }
-          }
-          pb = pn;
-          for (int k0 = 0; k0 < total; k0 += 32) {
-            const int k = k0 + lane;
-            int L = 0;  // the cell lane whose range [excl, incl) holds k
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1) {
-              const int e = __shfl_sync(FULL, excl, L + st);
-              if (L + st < 27 && e <= k) L += st;
-            }
-            const int w = __shfl_sync(FULL, want, L);
-            const int at = __shfl_sync(FULL, start, L) + k - __shfl_sync(FULL, excl, L);
-            int j = -1;
-            float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-            bool aj = false;
-            if (k < total) {
-              j = S.sorted[at];
-              if (S.ckey[j] != w) j = -1;
-              if (j >= 0) {
-                y = pos[j];
-                aj = S.amphi[j] != 0;
-              }
-            }
-            for (int g = 0; g < n_b; ++g) {
-              const int id = __shfl_sync(FULL, mine_i, g);
-              const float4 xi = pos[id];
-              const float d0 = y.x - xi.x, d1 = y.y - xi.y, d2 = y.z - xi.z;
-              const float r2 = __fmaf_rn(d2, d2, __fmaf_rn(d0, d0, __fmul_rn(d1, d1)));
-              const bool in = j >= 0 && j != id && r2 <= rv2;
-              const unsigned mk = __ballot_sync(FULL, in);
-              if (mk == 0) continue;
-              const int q = __shfl_sync(FULL, acc, g) + __popc(mk & lt);
-              const bool bb = aj && S.amphi[id] != 0;
-              const bool put = in && q < a.max_nb;
-              if (put)
-                a.nlist[static_cast<size_t>(q) * a.n_mono_total + b + id] = b + j;
-              const bool keep = put && !(r2 > (bb ? keep_bb : keep_aa));
-              const unsigned entry = static_cast<unsigned>(j) | (bb ? 0x8000u : 0u);
-              if (KMAX == 1 || lk == 0) {
-                const unsigned kk = __ballot_sync(FULL, keep);
-                const int t = __shfl_sync(FULL, kept, g) + __popc(kk & lt);
-                if (keep && t < ROWS) S.ent[t * NT + id] = static_cast<unsigned short>(entry);
-                if (lane == g) kept += __popc(kk);
-              } else if (put && (q >> lk) < ROWS) {
-                // by its place in the bead's list, which says whose it is;
-                // the threads close the gaps afterwards
-                S.ent[(q >> lk) * NT + ((id << lk) | (q & kmask))] =
-                    static_cast<unsigned short>(keep ? entry : MD_NO_ENTRY);
-              }
-              if (lane == g) acc += __popc(mk);
-            }
-          }
-          if (mine_i >= 0) {
-            int full = acc;
-            if (full > a.max_nb) {
-              raise_error(a.err, ERR_NEIGHBOR_OVF, static_cast<uint32_t>(b + mine_i),
-                          static_cast<uint32_t>(full));
-              full = a.max_nb;
-            }
-            a.ncount[b + mine_i] = full;
-            S.n_ent[mine_i] = static_cast<unsigned short>(KMAX == 1 || lk == 0 ? kept : full);
-          }
-        }
-      }
-      __syncthreads();
-      n_ent = mine ? S.n_ent[i] : 0;
-      if (KMAX > 1 && lk > 0) {  // this thread's share of the bead's list, gaps closed
-        const int rows = mine ? (n_ent - sub + kmask) >> lk : 0;
-        n_ent = rows > ROWS ? rows : 0;
-        for (int t = 0; t < rows && rows <= ROWS; ++t) {
-          const unsigned short e = S.ent[t * NT + tid];
-          if (e != MD_NO_ENTRY) S.ent[n_ent++ * NT + tid] = e;
-        }
-      }
+      n_ent = md_fast_build<NT, KMAX, ROWS>(a.nlist + b, a.ncount + b, a.n_mono_total, a.max_nb,
+                                            a.err, b, n, lk, step & 1, rv, keep_bb, keep_aa);
       fits = !__syncthreads_or(n_ent > ROWS);
-    } else if (n_ent < 0) {  // the lists of an earlier launch
-      n_ent = 0;
-      if (mine) {
-        const int cnt = a.ncount[b + i];
-        const int* nl = a.nlist + b + i;
-        const size_t stride = static_cast<size_t>(a.n_mono_total);
-        const bool ai = S.amphi[i] != 0;
-        constexpr int PF = 4;
-        for (int q0 = sub; q0 < cnt; q0 += PF << lk) {
-          int js[PF];
-#pragma unroll
-          for (int u = 0; u < PF; ++u) {
-            const int q = q0 + (u << lk);
-            js[u] = q < cnt ? nl[static_cast<size_t>(q) * stride] - b : -1;
-          }
-#pragma unroll
-          for (int u = 0; u < PF; ++u) {
-            const int j = js[u];
-            if (j < 0) continue;
-            const float4 y = S.ref[j];
-            const float d0 = y.x - xv[0], d1 = y.y - xv[1], d2 = y.z - xv[2];
-            const bool bb = ai && S.amphi[j] != 0;
-            if (!((d0 * d0 + d1 * d1) + d2 * d2 > (bb ? keep_bb : keep_aa))) {
-              if (n_ent < ROWS)
-                S.ent[n_ent * NT + tid] = static_cast<unsigned short>(j | (bb ? 0x8000 : 0));
-              ++n_ent;
-            }
-          }
-        }
-      }
+    } else if (n_ent < 0) {
+      n_ent = md_fast_take<NT, KMAX, ROWS>(a.nlist + b, a.ncount + b, a.n_mono_total, b, n, lk, keep_bb,
+                                           keep_aa);
       fits = !__syncthreads_or(n_ent > ROWS);
     }
     const bool want_epot = a.calc_epot && (step == total_steps - 1);
     // forces (Box.cpp:243-286)
     float F0 = 0.0f, F1 = 0.0f, F2 = 0.0f;
-    if (fits) {
-      // every bond end by a thread of its own, for the lead lanes below
-      for (int e = tid; e < n_bond; e += NT) {
-        const unsigned bd = S.bond[e];
-        const int j = static_cast<int>(bd & 0x7FFFu), ib = S.bead[e];
-        const float4 xb = pos[ib];
-        const float xx[3] = {xb.x, xb.y, xb.z};
-        float d[3], r2;
-        const bool anch = (bd & 0x8000u) != 0;
-        const float fa = md_bond_f32(a, pot, anch, pos[j], xx, d, &r2, b + ib, b + j);
-        if (want_epot) epot += md_fene_epot<float>(anch, r2);
-        S.bf[e] = make_float4(d[0], d[1], d[2], fa);
-      }
-      // Pairs, four at a time: their loads and arithmetic overlap (out of range
-      // the force is zero), the sums stay in list order.
-      for (int t0 = 0; t0 < n_ent; t0 += 4) {
-        float d0[4], d1[4], d2[4], fa[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = t0 + u < n_ent ? t0 + u : t0;
-          const unsigned e = S.ent[t * NT + tid];
-          const float4 y = pos[e & 0x7FFFu];
-          d0[u] = y.x - x[0];
-          d1[u] = y.y - x[1];
-          d2[u] = y.z - x[2];
-          const float r2 = (d0[u] * d0[u] + d1[u] * d1[u]) + d2[u] * d2[u];
-          fa[u] = pair_force_all(pot, (e & 0x8000u) != 0, r2, lambda, t0 + u < n_ent);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          F0 -= d0[u] * fa[u];
-          F1 -= d1[u] * fa[u];
-          F2 -= d2[u] * fa[u];
-        }
-      }
-      if (want_epot)
-        for (int t = 0; t < n_ent; ++t) {
-          const unsigned e = S.ent[t * NT + tid];
-          const float4 y = pos[e & 0x7FFFu];
-          const float d0 = y.x - x[0], d1 = y.y - x[1], d2 = y.z - x[2];
-          epot += md_pair_epot<float>(pot, (e & 0x8000u) != 0, (d0 * d0 + d1 * d1) + d2 * d2, lambda);
-        }
+    if (fits && !want_epot) {
+      if (pot == POT_REF4824)
+        md_fast_forces<NT, ROWS, POT_REF4824, U>(S, a, b, pos, n_bond, n_ent, x, lambda, F0, F1, F2);
+      else
+        md_fast_forces<NT, ROWS, POT_LJ126, U>(S, a, b, pos, n_bond, n_ent, x, lambda, F0, F1, F2);
       __syncthreads();  // the bonds are computed
       if (mine && lead) {  // then added, in order
         const int e1 = S.bstart[i + 1];
