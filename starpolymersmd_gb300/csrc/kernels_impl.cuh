@@ -21,11 +21,11 @@ int collide_cells_per_tile<Real>() {
   return SMPC_COLLIDE_CT;
 }
 
-template <>
-void launch_cycle_begin<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, int n_adv,
-                              double adv_scale, int gen_shift, cudaStream_t st) {
-  k_cycle_begin<Real><<<(n_rep + 127) / 128, 128, 0, st>>>(reps, dyn, n_rep, n_adv, adv_scale,
-                                                           gen_shift);
+template <typename R>
+static void launch_cycle_begin(const RepInfo* reps, RepDyn* dyn, int n_rep, int n_adv,
+                               double adv_scale, int gen_shift, cudaStream_t st) {
+  k_cycle_begin<R><<<(n_rep + 127) / 128, 128, 0, st>>>(reps, dyn, n_rep, n_adv, adv_scale,
+                                                        gen_shift);
 }
 
 template <>
@@ -48,10 +48,17 @@ template <>
 void launch_mono_prep<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, Real* mpos, Real* mvel,
                             uint2* mkey, int* mimg, uint32_t* count, ErrorState* err,
                             int mono_bin, int strict, FrameF* frames, double rot_c, double rot_s,
-                            int chunks, cudaStream_t st) {
+                            int chunks, int n_adv, double adv_scale, int gen_shift,
+                            cudaStream_t st) {
+  // CTAs of one replica must not race on its delrx: k_cycle_begin first
+  if (chunks > 1 && (n_adv > 0 || gen_shift)) {
+    launch_cycle_begin<Real>(reps, dyn, n_rep, n_adv, adv_scale, gen_shift, st);
+    n_adv = gen_shift = 0;
+  }
   const dim3 grid(n_rep, chunks > 0 ? chunks : 1);
-  k_mono_prep<Real, 256><<<grid, 256, 0, st>>>(reps, dyn, mpos, mvel, mkey, mimg, count, err,
-                                               mono_bin, strict, frames, rot_c, rot_s);
+  k_mono_prep<Real, 512><<<grid, 512, 0, st>>>(reps, dyn, mpos, mvel, mkey, mimg, count, err,
+                                               mono_bin, strict, frames, rot_c, rot_s, n_adv,
+                                               adv_scale, gen_shift);
 }
 
 #if SMPC_FAST_F32

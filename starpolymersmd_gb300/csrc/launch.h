@@ -62,13 +62,10 @@ struct CollideArgs {
 // Tile geometry chosen per precision (register budget of k_collide).
 template <typename R>
 int collide_cells_per_tile();
-int fluid_slots_per_tile(bool fp64);
+int fluid_slots_per_tile(bool fp64, long long slots);
 int temperature_cells_per_tile();
 int md_max_monomers();
 
-template <typename R>
-void launch_cycle_begin(const RepInfo* reps, RepDyn* dyn, int n_rep, int n_adv, double adv_scale,
-                        int gen_shift, cudaStream_t st);
 template <typename R>
 void launch_cycle_end(RepDyn* dyn, int n_rep, cudaStream_t st);
 template <typename R>
@@ -79,7 +76,8 @@ constexpr int INIT_PART_DOUBLES = 3 * 256;  // k_init_velocity_sum partials (INI
 template <typename R>
 void launch_mono_prep(const RepInfo* reps, RepDyn* dyn, int n_rep, R* mpos, R* mvel, uint2* mkey,
                       int* mimg, uint32_t* count, ErrorState* err, int mono_bin, int strict,
-                      FrameF* frames, double rot_c, double rot_s, int chunks, cudaStream_t st);
+                      FrameF* frames, double rot_c, double rot_s, int chunks, int n_adv, double adv_scale,
+                      int gen_shift, cudaStream_t st);
 template <typename R>
 void launch_fluid_bin(const Tile* tiles, int n_tiles, const RepInfo* reps, const RepDyn* dyn,
                       const FrameF* frames, const R* rec, uint2* keys, uint32_t* count,
@@ -173,7 +171,8 @@ template <typename R>
 void launch_pack_monomers(const R* mpos, const R* mvel, const R* mfrc, int n, double* pos,
                           double* vel, double* frc, cudaStream_t st);
 
-void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, uint32_t* grand, int n_cells,
+// tile_sum: scan_tile_count(n_cells) words
+void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, int n_cells,
                  cudaStream_t st);
 int scan_tile_count(int n_cells);
 void launch_build_perm(const uint2* keys, int n_slots, const uint2* mkey, int n_mono,

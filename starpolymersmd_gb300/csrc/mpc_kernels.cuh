@@ -2,8 +2,8 @@
 // R (double for the FP64 reference-parity path, float for the fast path).
 //
 // One collision (MPC::step, star-polymers/lib/Hydrodynamics/MPC.cpp:116-142):
-//   k_cycle_begin  delrx advance (MPC.cpp:117-118) + Philox grid shift   [graph mode]
-//   k_mono_prep    check_bounds recentring (MPC.cpp:160-190), monomer grid shift
+//   k_mono_prep    delrx advance (MPC.cpp:117-118) + Philox grid shift   [graph mode],
+//                  check_bounds recentring (MPC.cpp:160-190), monomer grid shift
 //                  (MPC.cpp:306-310) and monomer binning (MPC.cpp:221-236)
 //   k_fluid_bin    recentre/stream/shift/LE-wrap each solvent particle
 //                  (MPC.cpp:183-197, 301-305, 421-429) and bin it: cell key and
@@ -89,6 +89,19 @@ template <>
 __device__ __forceinline__ double make_slot_id<double>(uint32_t id) {
   return __longlong_as_double(static_cast<long long>(id));
 }
+
+// A float as a double without a conversion instruction (those issue on the
+// narrow FP64 pipe): the exponent rebiased and the mantissa moved; zeros,
+// subnormals, infinities and NaNs take the conversion, out of line.
+static __device__ __noinline__ double to_d_special(float x) { return static_cast<double>(x); }
+__device__ __forceinline__ double to_d(float x) {
+  const uint32_t b = __float_as_uint(x), e = (b >> 23) & 255u;
+  if (e - 1u >= 254u) return to_d_special(x);
+  return __hiloint2double(static_cast<int>((b & 0x80000000u) |
+                                           (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)),
+                          static_cast<int>(b << 29));
+}
+__device__ __forceinline__ double to_d(double x) { return x; }
 
 // ------------------------------------------------------- box geometry
 
@@ -362,32 +375,50 @@ __device__ __forceinline__ uint32_t warp_rank(uint32_t* count, uint32_t key) {
 
 // ------------------------------------------------------------ kernels
 
-// Graph mode: advance delrx n_sub times exactly as MPC.cpp:117-118 does on
-// every MD step, draw this collision's grid shift from Philox, and latch the
-// collision counter. One thread per replica.
+// delrx after n_adv MD steps, advanced on each exactly as MPC.cpp:117-118 does.
+// wrap_d takes the image from the magnitude bits: ten divisions and roundings
+// one after the other were 5 of the kernel's 8 us.
+__device__ __forceinline__ double advance_delrx(const RepInfo& ri, double d, int n_adv,
+                                                double adv_scale) {
+  const double Lx = static_cast<double>(ri.L[0]), half = Lx * 0.5;
+  const long long lo = __double_as_longlong(half * (1.0 - 0x1.0p-50)),
+                  hf = __double_as_longlong(half),
+                  far = __double_as_longlong(3.0 * half * (1.0 - 0x1.0p-50));
+  const double adv = __dmul_rn(__dmul_rn(ri.shear, static_cast<double>(ri.L[1])),
+                               __dmul_rn(ri.h, adv_scale));
+  for (int s = 0; s < n_adv; ++s) d = wrap_d(__dadd_rn(d, adv), Lx, lo, hf, far);
+  return d;
+}
+
+// This collision's grid shift: components 0 and 1 (pair 0) or 2 (pair 1) of
+// the replica's Philox draws at the collision counter.
+__device__ __forceinline__ Uniform2<double> draw_shift(const RepInfo& ri, unsigned long long step,
+                                                       unsigned pair) {
+  Uniform2<double> u = philox_uniforms<double>(ri.seed, 0xFFFFFFFFu, step, pair);
+  u.a -= 0.5;
+  u.b -= 0.5;
+  return u;
+}
+
+// Graph mode: advance delrx and draw the grid shift, for contexts that spread a
+// replica's monomers over several CTAs (elsewhere k_mono_prep does it itself).
+// One thread per replica.
 template <typename R>
 __global__ void k_cycle_begin(const RepInfo* reps, RepDyn* dyn, int n_rep, int n_adv,
                               double adv_scale, int gen_shift) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n_rep) return;
-  const RepInfo ri = reps[r];
+  const RepInfo& ri = reps[r];
   RepDyn& dn = dyn[r];
-  double d = dn.delrx;
-  const double Lx = static_cast<double>(ri.L[0]);
-  const double adv_dt = __dmul_rn(ri.h, adv_scale);
-  if (n_adv > 0) dn.h = ri.h;
-  for (int s = 0; s < n_adv; ++s) {
-    d = __dadd_rn(d, __dmul_rn(__dmul_rn(ri.shear, static_cast<double>(ri.L[1])), adv_dt));
-    d = __dsub_rn(d, __dmul_rn(Lx, round(__ddiv_rn(d, Lx))));
+  if (n_adv > 0) {
+    dn.h = ri.h;
+    dn.delrx = advance_delrx(ri, dn.delrx, n_adv, adv_scale);
   }
-  dn.delrx = d;
   if (gen_shift) {
-    const unsigned long long step = dn.step;
-    const Uniform2<double> a = philox_uniforms<double>(ri.seed, 0xFFFFFFFFu, step, 0u);
-    const Uniform2<double> b = philox_uniforms<double>(ri.seed, 0xFFFFFFFFu, step, 1u);
-    dn.shift[0] = a.a - 0.5;
-    dn.shift[1] = a.b - 0.5;
-    dn.shift[2] = b.a - 0.5;
+    const Uniform2<double> a = draw_shift(ri, dn.step, 0u), b = draw_shift(ri, dn.step, 1u);
+    dn.shift[0] = a.a;
+    dn.shift[1] = a.b;
+    dn.shift[2] = b.a;
   }
 }
 
@@ -501,92 +532,117 @@ __global__ void k_init_velocity_finish(const RepInfo* reps, int rep, R* st, cons
   }
 }
 
-// One CTA per replica: MPC::check_bounds, then shift and bin the monomers.
-// A replica that cannot recentre (mol0_size == 0, e.g. a periodic box) has
-// independent monomers: it is split over the gridDim.y CTAs of its row.
+// One CTA per replica: the delrx advance and the grid shift of this collision
+// (n_adv > 0, gen_shift: see k_cycle_begin), MPC::check_bounds, then shift and
+// bin the monomers. A replica that cannot recentre (mol0_size == 0, e.g. a
+// periodic box) has independent monomers: it is split over the gridDim.y CTAs
+// of its row.
+//
+// A chain of latencies, so what is independent runs beside it: the advance,
+// the draws and the frame record are one thread's work each, in warps of their
+// own. Per-replica values go through shared memory instead of global memory
+// and back. Recentring in FP32 gives each of the six sums a warp whose lanes
+// add 1/32 of the beads, where all warps of the block issued six butterflies
+// on the FP64 pipe. Together with k_cycle_begin 20 us before, 10.7 now (one star
+// of 121 beads that recentres).
 template <typename R, int NT>
 __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* dyn, R* mpos,
                                                   R* mvel, uint2* mkey, int* mimg,
                                                   uint32_t* count, ErrorState* err,
                                                   int mono_bin, int strict, FrameF* frames,
-                                                  double rot_c, double rot_s) {
+                                                  double rot_c, double rot_s, int n_adv,
+                                                  double adv_scale, int gen_shift) {
+  static_assert(NT >= 192, "six warps sum the recentring");
   const int r = blockIdx.x;
-  const RepInfo ri = reps[r];
+  const RepInfo& ri = reps[r];
   const bool split = ri.mol0_size == 0;
   if (blockIdx.y > 0 && !split) return;
-  __shared__ int s_out;
-  if (threadIdx.x == 0) s_out = 0;
-  __syncthreads();
+  __shared__ double s_delrx, s_h, s_shift[3], s_com[6];
+  RepDyn& dn = dyn[r];
+  const int tid = static_cast<int>(threadIdx.x);
+  if (tid == 0) {
+    double d = dn.delrx, h = dn.h;
+    if (n_adv > 0) {
+      h = ri.h;
+      d = advance_delrx(ri, d, n_adv, adv_scale);
+      dn.h = h;
+      dn.delrx = d;
+    }
+    s_delrx = d;
+    s_h = h;
+  } else if (tid == 32 || tid == 64) {
+    const int q = tid >> 5;  // 1: components 0 and 1, 2: component 2
+    if (gen_shift) {
+      const Uniform2<double> u = draw_shift(ri, dn.step, static_cast<unsigned>(q - 1));
+      s_shift[2 * q - 2] = dn.shift[2 * q - 2] = u.a;
+      if (q == 1) s_shift[1] = dn.shift[1] = u.b;
+    } else {
+      s_shift[2 * q - 2] = dn.shift[2 * q - 2];
+      if (q == 1) s_shift[1] = dn.shift[1];
+    }
+  } else if (tid >= 96 && tid < 102) {
+    const int q = tid - 96;
+    s_com[q] = q < 3 ? dn.com[q] : dn.comv[q - 3];
+  }
   const int per = split ? (ri.n_mono + gridDim.y - 1) / gridDim.y : ri.n_mono;
   const int b = ri.mono_base + static_cast<int>(blockIdx.y) * per;
   const int n = max(0, min(per, ri.n_mono - static_cast<int>(blockIdx.y) * per));
   // MPC.cpp:166: any monomer with |x_d| >= L_d/2 - 0.5 triggers recentring
-  for (int i = threadIdx.x; i < n && !split; i += NT) {
+  int over = 0;
+  for (int i = tid; i < n && !split; i += NT) {
     const R4<R> x = ld4_rw(mpos, b + i);
     const R xs[3] = {x.x, x.y, x.z};
     for (int d = 0; d < 3; ++d)
-      if (r_fabs(xs[d]) >= (static_cast<R>(ri.L[d]) * R(0.5) - R(0.5))) s_out = 1;
+      if (r_fabs(xs[d]) >= (static_cast<R>(ri.L[d]) * R(0.5) - R(0.5))) over = 1;
   }
-  __syncthreads();
-  RepDyn& dn = dyn[r];
-  const int out = s_out && ri.mol0_size > 0;
-  if (!std::is_same<R, double>::value && out) {
-    // fast path: block-parallel centre of mass (FP64 sums, order free)
-    __shared__ double s_c[6];
-    if (threadIdx.x < 6) s_c[threadIdx.x] = 0.0;
+  const int out = __syncthreads_or(over) && ri.mol0_size > 0;
+  if (out) {
+    // Molecule::calculate_center_of_mass[_velocity] (Molecule.cpp:139-155)
+    // over molecule 0: sum q by warp q (FP32: FP64 sums, order free) or by
+    // lane q (FP64: sequential sums, as the reference does)
+    const bool seq = std::is_same<R, double>::value;
+    const int q = seq ? tid : tid >> 5;
+    if (q < 6) {
+      const R* src = (q < 3 ? mpos : mvel) + 4 * static_cast<size_t>(b) + (q < 3 ? q : q - 3);
+      double c = 0.0;
+      if (seq) {
+#pragma unroll 8
+        for (int i = 0; i < ri.mol0_size; ++i) c = __dadd_rn(c, to_d(src[4 * i]));
+      } else {
+        for (int i = tid & 31; i < ri.mol0_size; i += 32) c += to_d(src[4 * i]);
+        for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xFFFFFFFFu, c, o);
+      }
+      if (seq || (tid & 31) == 0) {
+        c = __ddiv_rn(c, static_cast<double>(ri.mol0_size));
+        s_com[q] = c;
+        (q < 3 ? dn.com[q] : dn.comv[q - 3]) = c;
+      }
+    }
     __syncthreads();
-    double c[6] = {0, 0, 0, 0, 0, 0};
-    for (int i = threadIdx.x; i < ri.mol0_size; i += NT) {
-      const R4<R> x = ld4_rw(mpos, b + i);
-      const R4<R> v = ld4_rw(mvel, b + i);
-      c[0] += x.x; c[1] += x.y; c[2] += x.z;
-      c[3] += v.x; c[4] += v.y; c[5] += v.z;
-    }
-    for (int q = 0; q < 6; ++q) {
-      double t = c[q];
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, o);
-      if ((threadIdx.x & 31) == 0) atomicAdd(&s_c[q], t);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      dn.recentre = 1;
-      const double nm = static_cast<double>(ri.mol0_size);
-      for (int d = 0; d < 3; ++d) {
-        dn.com[d] = s_c[d] / nm;
-        dn.comv[d] = s_c[3 + d] / nm;
-      }
-    }
-  } else if (threadIdx.x == 0 && blockIdx.y == 0) {
-    dn.recentre = out;
-    if (out) {
-      // Molecule::calculate_center_of_mass[_velocity] (Molecule.cpp:139-155):
-      // sequential sums over molecule 0, as the reference does.
-      double c[3] = {0, 0, 0}, cv[3] = {0, 0, 0};
-      for (int i = 0; i < ri.mol0_size; ++i) {
-        const R4<R> x = ld4_rw(mpos, b + i);
-        const R4<R> v = ld4_rw(mvel, b + i);
-        c[0] = __dadd_rn(c[0], static_cast<double>(x.x));
-        c[1] = __dadd_rn(c[1], static_cast<double>(x.y));
-        c[2] = __dadd_rn(c[2], static_cast<double>(x.z));
-        cv[0] = __dadd_rn(cv[0], static_cast<double>(v.x));
-        cv[1] = __dadd_rn(cv[1], static_cast<double>(v.y));
-        cv[2] = __dadd_rn(cv[2], static_cast<double>(v.z));
-      }
-      const double nm = static_cast<double>(static_cast<unsigned>(ri.mol0_size));
-      for (int d = 0; d < 3; ++d) {
-        dn.com[d] = __ddiv_rn(c[d], nm);
-        dn.comv[d] = __ddiv_rn(cv[d], nm);
-      }
+  }
+  // One thread converts: in all of them the same FP64 instructions kept the
+  // narrow pipe busy for longer than the rest of the block's work.
+  __shared__ Geo<R> s_geo;
+  RepDyn now;
+  if (tid == 0 || tid == NT - 32) {  // for make_geo; for the frame record
+    now.delrx = s_delrx;
+    now.h = s_h;
+    now.recentre = out;
+    for (int d = 0; d < 3; ++d) {
+      now.shift[d] = s_shift[d];
+      now.com[d] = s_com[d];
+      now.comv[d] = s_com[3 + d];
     }
   }
+  if (tid == 0) {
+    if (blockIdx.y == 0) dn.recentre = out;
+    s_geo = make_geo<R>(ri, now, mono_bin);
+  }
   __syncthreads();
-  const Geo<R> g = make_geo<R>(ri, dn, mono_bin);
-  const R s0 = static_cast<R>(dn.shift[0]), s1 = static_cast<R>(dn.shift[1]),
-          s2 = static_cast<R>(dn.shift[2]);
-  const R c0 = static_cast<R>(dn.com[0]), c1 = static_cast<R>(dn.com[1]),
-          c2 = static_cast<R>(dn.com[2]);
-  const R cv0 = static_cast<R>(dn.comv[0]), cv1 = static_cast<R>(dn.comv[1]),
-          cv2 = static_cast<R>(dn.comv[2]);
+  const Geo<R>& g = s_geo;
+  const R s0 = g.shift[0], s1 = g.shift[1], s2 = g.shift[2];
+  const R c0 = g.com[0], c1 = g.com[1], c2 = g.com[2];
+  const R cv0 = g.comv[0], cv1 = g.comv[1], cv2 = g.comv[2];
   const int iters = (n + NT - 1) / NT;
   for (int it = 0; it < iters; ++it) {
     const int i = it * NT + threadIdx.x;
@@ -624,20 +680,20 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
       mimg[b + i] = img;
     }
   }
-  if (frames != nullptr && threadIdx.x == 0 && blockIdx.y == 0) {
+  if (frames != nullptr && tid == NT - 32 && blockIdx.y == 0) {
     FrameF f;
     for (int d = 0; d < 3; ++d) {
       f.L[d] = static_cast<float>(ri.L[d]);
       f.half[d] = 0.5f * static_cast<float>(ri.L[d]);
       f.Li[d] = ri.L[d];
-      f.shift[d] = static_cast<float>(dn.shift[d]);
-      f.com[d] = static_cast<float>(dn.com[d]);
-      f.comv[d] = static_cast<float>(dn.comv[d]);
+      f.shift[d] = static_cast<float>(now.shift[d]);
+      f.com[d] = static_cast<float>(now.com[d]);
+      f.comv[d] = static_cast<float>(now.comv[d]);
     }
     f.shear = static_cast<float>(ri.shear);
     f.shearLy = static_cast<float>(ri.shear * ri.L[1]);
-    f.delrx = static_cast<float>(dn.delrx);
-    f.h = static_cast<float>(dn.h);
+    f.delrx = static_cast<float>(now.delrx);
+    f.h = static_cast<float>(now.h);
     f.kT = static_cast<float>(ri.kT);
     f.solvent_mass = static_cast<float>(ri.solvent_mass);
     f.rot_c = static_cast<float>(rot_c);
@@ -681,8 +737,12 @@ __global__ void __launch_bounds__(NT) k_fluid_bin(const Tile* tiles, const RepIn
   constexpr int U = std::is_same<R, double>::value ? 2 : 4;
   const Tile t = tiles[blockIdx.x];
   const RepInfo& ri = reps[t.rep];
-  const RepDyn dn = dyn[t.rep];
-  const Geo<R> g = make_geo<R>(ri, dn, 0);
+  // one thread's FP64 arithmetic and conversions (a tenth of the FP64 kernel
+  // when every thread repeated them)
+  __shared__ Geo<R> s_geo;
+  if (threadIdx.x == 0) s_geo = make_geo<R>(ri, dyn[t.rep], 0);
+  __syncthreads();
+  const Geo<R> g = s_geo;
   const uint32_t cbase = static_cast<uint32_t>(ri.cell_base);
   const uint32_t ncell = static_cast<uint32_t>(ri.n_cell);
   const unsigned lane = threadIdx.x & 31u;
@@ -1118,8 +1178,9 @@ __global__ void __launch_bounds__(NT) k_collide(
   C.mvel = mvel;
   C.mkey = mkey;
   C.mimg = mimg;
+  __shared__ Geo<R> s_geo;
+  if (threadIdx.x == 0) s_geo = make_geo<R>(ri, dyn[t.rep], mono_bin);
   C.dn = dyn[t.rep];
-  C.g = make_geo<R>(ri, C.dn, mono_bin);
   C.solvent_mass = static_cast<R>(ri.solvent_mass);
   C.cbase = static_cast<uint32_t>(ri.cell_base);
   C.c0 = static_cast<uint32_t>(t.begin);
@@ -1133,6 +1194,7 @@ __global__ void __launch_bounds__(NT) k_collide(
 
   for (int i = threadIdx.x; i <= nc; i += NT) s_off[i] = off[t.begin + i];
   __syncthreads();
+  C.g = s_geo;
   const uint32_t p0 = s_off[0], p1 = s_off[nc];
   const int n = static_cast<int>(p1 - p0);
   const int nloc = n < CAP ? n : CAP;

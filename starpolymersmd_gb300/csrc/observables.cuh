@@ -27,19 +27,6 @@ namespace smpc {
 constexpr int OBS_PER_REP = 16;
 constexpr int UNWRAP_NT = 256;  // threads (and beads per chunk) of k_unwrap_molecules
 
-// A float as a double without a conversion instruction (those issue on the
-// narrow FP64 pipe): the exponent rebiased and the mantissa moved; zeros,
-// subnormals, infinities and NaNs take the conversion, out of line.
-static __device__ __noinline__ double to_d_special(float x) { return static_cast<double>(x); }
-__device__ __forceinline__ double to_d(float x) {
-  const uint32_t b = __float_as_uint(x), e = (b >> 23) & 255u;
-  if (e - 1u >= 254u) return to_d_special(x);
-  return __hiloint2double(static_cast<int>((b & 0x80000000u) |
-                                           (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u)),
-                          static_cast<int>(b << 29));
-}
-__device__ __forceinline__ double to_d(double x) { return x; }
-
 // Centre of molecule [b, e), unweighted mean position and velocity, summed in
 // monomer order like the reference. The block stages the monomers in shared
 // memory, then six lanes add one component each: one thread that loaded and

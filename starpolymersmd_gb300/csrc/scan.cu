@@ -3,9 +3,9 @@
 // replaces MPC::sort's vector<vector<MPCParticle*>> push_back cell lists
 // (star-polymers/lib/Hydrodynamics/MPC.cpp:201-237) with integer arithmetic.
 //
-// Scan: three launches over C cells: per-tile scan (2048 cells / CTA, count
-// is re-zeroed for the next collision while it is read), scan of the tile
-// totals (one CTA), add of the tile bases. off[C] receives the total.
+// Scan: two launches over C cells: per-tile scan (count is re-zeroed for the
+// next collision while it is read), then the totals of the tiles before are
+// added; one launch of one CTA for few cells. off[C] receives the total.
 #include <stdint.h>
 
 #include "launch.h"
@@ -17,56 +17,33 @@ constexpr int SCAN_NT = 256;
 constexpr int SCAN_IPT = 8;
 constexpr int SCAN_TILE = SCAN_NT * SCAN_IPT;
 
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
-  __shared__ uint32_t warp_sums[SCAN_NT / 32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warp_sums[w] = x;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t s = lane < SCAN_NT / 32 ? warp_sums[lane] : 0u;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-      if (lane >= o) s += y;
-    }
-    if (lane < SCAN_NT / 32) warp_sums[lane] = s;
-  }
-  __syncthreads();
-  const uint32_t before = (w > 0 ? warp_sums[w - 1] : 0u) + x - v;
-  *total = warp_sums[SCAN_NT / 32 - 1];
-  return before;
-}
-
 // One tile of SCAN_TILE cells per CTA. Warp w owns the tile's w-th run of
 // 32 * SCAN_IPT consecutive cells, read as SCAN_IPT rows of 32 (every load and
 // store of a warp is one contiguous 128-byte row); each row is a warp scan
 // carried into the next, then the warps' totals give each warp's base.
-__global__ void __launch_bounds__(SCAN_NT) k_scan_tiles(uint32_t* __restrict__ count,
-                                                        uint32_t* __restrict__ off,
-                                                        uint32_t* __restrict__ tile_sum, int n) {
-  __shared__ uint32_t warp_tot[SCAN_NT / 32];
+// Offsets are within the tile; k_scan_add adds the tiles before. A scan of one
+// tile is complete (one launch).
+template <int NT, int IPT>
+__global__ void __launch_bounds__(NT) k_scan_tiles(uint32_t* __restrict__ count,
+                                                   uint32_t* __restrict__ off,
+                                                   uint32_t* __restrict__ tile_sum, int n) {
+  __shared__ uint32_t warp_tot[NT / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int seg = blockIdx.x * SCAN_TILE + w * (32 * SCAN_IPT);
-  uint32_t c[SCAN_IPT], pre[SCAN_IPT];
+  const int seg = blockIdx.x * (NT * IPT) + w * (32 * IPT);
+  uint32_t c[IPT], pre[IPT];
 #pragma unroll
-  for (int k = 0; k < SCAN_IPT; ++k) {
+  for (int k = 0; k < IPT; ++k) {
     const int i = seg + 32 * k + lane;
     c[k] = i < n ? count[i] : 0u;
   }
 #pragma unroll
-  for (int k = 0; k < SCAN_IPT; ++k) {
+  for (int k = 0; k < IPT; ++k) {
     const int i = seg + 32 * k + lane;
     if (i < n) count[i] = 0u;  // re-zeroed for the next collision
   }
   uint32_t carry = 0;
 #pragma unroll
-  for (int k = 0; k < SCAN_IPT; ++k) {
+  for (int k = 0; k < IPT; ++k) {
     uint32_t x = c[k];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -80,64 +57,55 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_tiles(uint32_t* __restrict__ c
   __syncthreads();
   uint32_t wbase = 0, total = 0;
 #pragma unroll
-  for (int q = 0; q < SCAN_NT / 32; ++q) {
+  for (int q = 0; q < NT / 32; ++q) {
     const uint32_t t = warp_tot[q];
     if (q < w) wbase += t;
     total += t;
   }
 #pragma unroll
-  for (int k = 0; k < SCAN_IPT; ++k) {
+  for (int k = 0; k < IPT; ++k) {
     const int i = seg + 32 * k + lane;
     if (i < n) off[i] = wbase + pre[k];
   }
-  if (threadIdx.x == 0) tile_sum[blockIdx.x] = total;
-}
-
-// Exclusive scan of up to SCAN_TILE tile totals in one CTA.
-__global__ void __launch_bounds__(SCAN_NT) k_scan_tile_sums(uint32_t* __restrict__ tile_sum,
-                                                            int n_tiles,
-                                                            uint32_t* __restrict__ grand) {
-  uint32_t carry = 0;
-  for (int chunk = 0; chunk < n_tiles; chunk += SCAN_TILE) {
-    const int base = chunk + threadIdx.x * SCAN_IPT;
-    uint32_t c[SCAN_IPT];
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_IPT; ++k) {
-      c[k] = base + k < n_tiles ? tile_sum[base + k] : 0u;
-      s += c[k];
-    }
-    uint32_t total;
-    uint32_t run = block_exclusive_scan(s, &total) + carry;
-#pragma unroll
-    for (int k = 0; k < SCAN_IPT; ++k) {
-      if (base + k < n_tiles) tile_sum[base + k] = run;
-      run += c[k];
-    }
-    carry += total;
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    tile_sum[blockIdx.x] = total;
+    if (gridDim.x == 1) off[n] = total;
   }
-  if (threadIdx.x == 0) *grand = carry;
 }
 
-// SCAN_ADD_U cells per thread, a block apart (coalesced, independent loads)
-constexpr int SCAN_ADD_U = 4;
+// Adds the totals of the tiles before to a tile's offsets; every CTA sums them
+// for itself, beside its loads of the offsets, instead of waiting for a launch
+// that scans them. (A single launch with decoupled look-back, each tile polling
+// its predecessors' totals, took 9.3 us for 62 tiles and 67 for 3,907; the two
+// launches take 6.4 and 24, three with one for the totals took 9 and 28.)
 __global__ void __launch_bounds__(SCAN_NT) k_scan_add(uint32_t* __restrict__ off,
-                                                      const uint32_t* __restrict__ tile_base,
-                                                      const uint32_t* __restrict__ grand, int n) {
-  const int base = blockIdx.x * (SCAN_NT * SCAN_ADD_U) + threadIdx.x;
-  uint32_t v[SCAN_ADD_U];
+                                                      const uint32_t* __restrict__ tile_sum,
+                                                      int n) {
+  __shared__ uint32_t warp_tot[SCAN_NT / 32];
+  const int tile = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int base = tile * SCAN_TILE + threadIdx.x;
+  uint32_t v[SCAN_IPT];
 #pragma unroll
-  for (int u = 0; u < SCAN_ADD_U; ++u) {
+  for (int u = 0; u < SCAN_IPT; ++u) {
     const int i = base + u * SCAN_NT;
-    v[u] = i < n ? off[i] + tile_base[i / SCAN_TILE] : 0u;
+    v[u] = i < n ? off[i] : 0u;
   }
+  uint32_t before = 0;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < tile; t += SCAN_NT) before += tile_sum[t];
+  before = __reduce_add_sync(0xFFFFFFFFu, before);
+  if (lane == 0) warp_tot[w] = before;
+  __syncthreads();
+  before = 0;
 #pragma unroll
-  for (int u = 0; u < SCAN_ADD_U; ++u) {
+  for (int q = 0; q < SCAN_NT / 32; ++q) before += warp_tot[q];
+#pragma unroll
+  for (int u = 0; u < SCAN_IPT; ++u) {
     const int i = base + u * SCAN_NT;
-    if (i < n) off[i] = v[u];
-    if (i == n) off[n] = *grand;
+    if (i < n) off[i] = v[u] + before;
   }
+  if (tile == static_cast<int>(gridDim.x) - 1 && threadIdx.x == 0)
+    off[n] = before + tile_sum[tile];
 }
 
 // perm[off[cell] + rank] = source. Each thread takes PERM_U entries a block
@@ -229,16 +197,23 @@ __global__ void __launch_bounds__(PERM_NT) k_build_perm_packed(
   }
 }
 
+// Up to this many cells one CTA scans them all: 5.1 us for 8,000 cells, against
+// 6.5 and a launch more in two (8.5 in three, with one for the totals); with
+// four times as many cells per thread it took 12 us for 29,791.
+constexpr int SCAN_ONE_NT = 1024, SCAN_ONE_IPT = 8;
+constexpr int SCAN_ONE = SCAN_ONE_NT * SCAN_ONE_IPT;
 int scan_tile_count(int n_cells) { return (n_cells + SCAN_TILE - 1) / SCAN_TILE; }
 
-void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, uint32_t* grand,
-                 int n_cells, cudaStream_t st) {
+void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, int n_cells,
+                 cudaStream_t st) {
+  if (n_cells <= SCAN_ONE) {
+    k_scan_tiles<SCAN_ONE_NT, SCAN_ONE_IPT><<<1, SCAN_ONE_NT, 0, st>>>(count, off, tile_sum,
+                                                                       n_cells);
+    return;
+  }
   const int tiles = scan_tile_count(n_cells);
-  k_scan_tiles<<<tiles, SCAN_NT, 0, st>>>(count, off, tile_sum, n_cells);
-  k_scan_tile_sums<<<1, SCAN_NT, 0, st>>>(tile_sum, tiles, grand);
-  const int per_block = SCAN_NT * SCAN_ADD_U;
-  k_scan_add<<<(n_cells + 1 + per_block - 1) / per_block, SCAN_NT, 0, st>>>(off, tile_sum, grand,
-                                                                           n_cells);
+  k_scan_tiles<SCAN_NT, SCAN_IPT><<<tiles, SCAN_NT, 0, st>>>(count, off, tile_sum, n_cells);
+  k_scan_add<<<tiles, SCAN_NT, 0, st>>>(off, tile_sum, n_cells);
 }
 
 void launch_build_perm_packed(const Tile* tiles, int n_tiles, const RepInfo* reps,

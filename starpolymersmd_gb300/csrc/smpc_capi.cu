@@ -57,7 +57,6 @@ struct smpc_ctx {
   uint32_t* d_count = nullptr;
   uint32_t* d_off = nullptr;
   uint32_t* d_tsum = nullptr;
-  uint32_t* d_grand = nullptr;
 
   void* d_mpos = nullptr;
   void* d_mvel = nullptr;
@@ -220,27 +219,35 @@ void launch_permutation(smpc_ctx* ctx) {
 }
 
 template <typename R>
-int launch_binning(smpc_ctx* ctx, int cur) {
-  const int strict = ctx->opt.strict_cells;
-  const R* rec_in = static_cast<const R*>(ctx->d_rec[cur]);
+void launch_prep(smpc_ctx* ctx, int n_adv, double adv, int gen_shift) {
   smpc::launch_mono_prep<R>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, static_cast<R*>(ctx->d_mpos),
                             static_cast<R*>(ctx->d_mvel), ctx->d_mkey, ctx->d_mimg, ctx->d_count,
-                            ctx->d_err, ctx->opt.mono_bin, strict, ctx->d_frames, ctx->rot_c,
-                            ctx->rot_s, ctx->mono_chunks, ctx->st);
+                            ctx->d_err, ctx->opt.mono_bin, ctx->opt.strict_cells, ctx->d_frames,
+                            ctx->rot_c, ctx->rot_s, ctx->mono_chunks, n_adv, adv, gen_shift,
+                            ctx->st);
+}
+
+// n_adv > 0: delrx is advanced by that many MD steps of adv h each (graph mode);
+// gen_shift: the device draws the grid shift from this collision's counter
+template <typename R>
+int launch_binning(smpc_ctx* ctx, int cur, int n_adv, double adv, int gen_shift) {
+  const int strict = ctx->opt.strict_cells;
+  const R* rec_in = static_cast<const R*>(ctx->d_rec[cur]);
+  launch_prep<R>(ctx, n_adv, adv, gen_shift);
   smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
                             ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
                             ctx->opt.angular_momentum ? -1 : ctx->var_bin,
                             ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->st);
   ctx->frame_ok = ctx->d_frame != nullptr;
-  smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, ctx->d_grand,
-                    static_cast<int>(ctx->total_cells), ctx->st);
+  smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
+                    ctx->st);
   launch_permutation(ctx);
   return SMPC_OK;
 }
 
 template <typename R>
-int launch_collision(smpc_ctx* ctx, int rng, int cur) {
-  launch_binning<R>(ctx, cur);
+int launch_collision(smpc_ctx* ctx, int rng, int cur, int n_adv, double adv) {
+  launch_binning<R>(ctx, cur, n_adv, adv, rng == smpc::RNG_PHILOX ? 1 : 0);
   smpc::launch_collide<R>(collide_args<R>(ctx, rng, cur), ctx->st);
   return SMPC_OK;
 }
@@ -327,12 +334,8 @@ int profiled_cycle(smpc_ctx* ctx, int cur, cudaEvent_t* ev) {
   cudaEventRecord(ev[0], ctx->st);
   launch_md_steps<R>(ctx, nsub, 0, 0);
   cudaEventRecord(ev[1 + PH_MD], ctx->st);
-  smpc::launch_cycle_begin<R>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, nsub, adv, 1, ctx->st);
-  cudaEventRecord(ev[1 + PH_BEGIN], ctx->st);
-  smpc::launch_mono_prep<R>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, static_cast<R*>(ctx->d_mpos),
-                            static_cast<R*>(ctx->d_mvel), ctx->d_mkey, ctx->d_mimg, ctx->d_count,
-                            ctx->d_err, ctx->opt.mono_bin, strict, ctx->d_frames, ctx->rot_c,
-                            ctx->rot_s, ctx->mono_chunks, ctx->st);
+  cudaEventRecord(ev[1 + PH_BEGIN], ctx->st);  // the collision's begin is part of PH_MONO
+  launch_prep<R>(ctx, nsub, adv, 1);
   cudaEventRecord(ev[1 + PH_MONO], ctx->st);
   smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
                             ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
@@ -340,8 +343,8 @@ int profiled_cycle(smpc_ctx* ctx, int cur, cudaEvent_t* ev) {
                             ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->st);
   ctx->frame_ok = ctx->d_frame != nullptr;
   cudaEventRecord(ev[1 + PH_BIN], ctx->st);
-  smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, ctx->d_grand,
-                    static_cast<int>(ctx->total_cells), ctx->st);
+  smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
+                    ctx->st);
   cudaEventRecord(ev[1 + PH_SCAN], ctx->st);
   launch_permutation(ctx);
   cudaEventRecord(ev[1 + PH_PERM], ctx->st);
@@ -359,9 +362,8 @@ int record_cycle(smpc_ctx* ctx, int cur) {
   launch_md_steps<R>(ctx, nsub, 0, 0);
   double adv = 1.0;
   if (ctx->opt.delrx_mode == SMPC_DELRX_PHYSICAL) adv = 1.0 / nsub;
-  // h is per replica; k_cycle_begin advances delrx by shear*Ly*h*adv per MD step
-  smpc::launch_cycle_begin<R>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, nsub, adv, 1, ctx->st);
-  launch_collision<R>(ctx, smpc::RNG_PHILOX, cur);
+  // h is per replica; delrx advances by shear*Ly*h*adv per MD step
+  launch_collision<R>(ctx, smpc::RNG_PHILOX, cur, nsub, adv);
   smpc::launch_cycle_end<R>(ctx->d_dyn, ctx->n_rep, ctx->st);
   return SMPC_OK;
 }
@@ -662,7 +664,6 @@ int create_buffers(smpc_ctx* ctx) {
   CU(cudaMemset(ctx->d_count, 0, C * sizeof(uint32_t)));
   CU(dalloc(&ctx->d_off, C + 1));
   CU(dalloc(&ctx->d_tsum, static_cast<size_t>(smpc::scan_tile_count(static_cast<int>(C)))));
-  CU(dalloc(&ctx->d_grand, 1));
   CU(dalloc(&ctx->d_init_part, static_cast<size_t>(smpc::INIT_PART_DOUBLES)));
   CU(dalloc(reinterpret_cast<R**>(&ctx->d_mpos), 4 * M));
   CU(dalloc(reinterpret_cast<R**>(&ctx->d_mvel), 4 * M));
@@ -761,7 +762,7 @@ void free_all(smpc_ctx* ctx) {
   if (ctx->d_and_v) cudaFree(ctx->d_and_v);
   void* ptrs[] = {ctx->d_reps, ctx->d_dyn, ctx->d_bin_tiles, ctx->d_col_tiles, ctx->d_tmp_tiles,
                   ctx->d_tpart, ctx->d_keys, ctx->d_perm, ctx->d_count, ctx->d_off, ctx->d_tsum,
-                  ctx->d_grand, ctx->d_mpos, ctx->d_mvel, ctx->d_mfrc, ctx->d_mver, ctx->d_mkey,
+                  ctx->d_mpos, ctx->d_mvel, ctx->d_mfrc, ctx->d_mver, ctx->d_mkey,
                   ctx->d_mimg, ctx->d_bond_start, ctx->d_bonds, ctx->d_nlist, ctx->d_ncount,
                   ctx->d_md_order, ctx->d_inj, ctx->d_err, ctx->d_frames, ctx->d_rep_mols,
                   ctx->d_mols, ctx->d_obs, ctx->d_prof, ctx->d_c6, ctx->d_dstage, ctx->d_mol_obs,
@@ -778,7 +779,7 @@ void free_all(smpc_ctx* ctx) {
 
 template <typename R>
 int dispatch_collision(smpc_ctx* ctx, int rng) {
-  launch_collision<R>(ctx, rng, ctx->cur);
+  launch_collision<R>(ctx, rng, ctx->cur, 0, 0.0);
   if (rng == SMPC_RNG_PHILOX) smpc::launch_cycle_end<R>(ctx->d_dyn, ctx->n_rep, ctx->st);
   ctx->cur ^= 1;
   ctx->collided = true;
@@ -1114,7 +1115,7 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
   const int ct = opt->precision == SMPC_FP64 ? smpc::collide_cells_per_tile<double>()
                                              : smpc::collide_cells_per_tile<float>();
   std::vector<Tile> bin =
-      make_tiles(ctx->reps, false, smpc::fluid_slots_per_tile(opt->precision == SMPC_FP64));
+      make_tiles(ctx->reps, false, smpc::fluid_slots_per_tile(opt->precision == SMPC_FP64, ctx->total_slots));
   std::vector<Tile> col;
   if (fast_path(ctx)) {
     for (const RepInfo& ri : ctx->reps) {
@@ -1371,13 +1372,6 @@ int smpc_mpc_step(smpc_ctx* ctx, long t, double dt, const smpc_inject* inj) {
     CU(cudaMemcpyAsync(ctx->d_inj + 2 * C, inj->u_theta, C * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
   }
   if (int rc = upload_host_dyn(ctx)) return rc;
-  if (rng == SMPC_RNG_PHILOX) {
-    // device draws the shift from this collision's counter
-    if (ctx->opt.precision == SMPC_FP64)
-      smpc::launch_cycle_begin<double>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, 0, 0.0, 1, ctx->st);
-    else
-      smpc::launch_cycle_begin<float>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, 0, 0.0, 1, ctx->st);
-  }
   int rc = ctx->opt.precision == SMPC_FP64 ? dispatch_collision<double>(ctx, rng)
                                            : dispatch_collision<float>(ctx, rng);
   if (rc) return rc;
@@ -1407,16 +1401,10 @@ int smpc_mpc_bin(smpc_ctx* ctx, long t, double dt, const double* shift, int* col
     return fail(ctx, SMPC_E_ARG, "inject mode needs the grid shift");
   }
   if (int rc = upload_host_dyn(ctx)) return rc;
-  if (!shift) {
-    if (ctx->opt.precision == SMPC_FP64)
-      smpc::launch_cycle_begin<double>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, 0, 0.0, 1, ctx->st);
-    else
-      smpc::launch_cycle_begin<float>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, 0, 0.0, 1, ctx->st);
-  }
   if (ctx->opt.precision == SMPC_FP64)
-    launch_binning<double>(ctx, ctx->cur);
+    launch_binning<double>(ctx, ctx->cur, 0, 0.0, shift == nullptr);
   else
-    launch_binning<float>(ctx, ctx->cur);
+    launch_binning<float>(ctx, ctx->cur, 0, 0.0, shift == nullptr);
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(ctx->st));
   ctx->binned = true;
