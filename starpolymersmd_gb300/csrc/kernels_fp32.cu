@@ -4,6 +4,7 @@
 #define SMPC_COLLIDE_NT 256
 #define SMPC_COLLIDE_CT 128
 #define SMPC_COLLIDE_CAP 1408
+#define SMPC_COLLIDE_BLOCKS 3
 #define SMPC_BIN_NT 256
 #define SMPC_MD_NT 1024
 #define SMPC_MD_MPT 1

@@ -1,10 +1,12 @@
 // FP64 reference-parity instantiation. Built with -fmad=false so every
-// multiply and add rounds separately, in the reference's order.
+// multiply and add rounds separately, in the reference's order; only the
+// collision itself (cell sums, rotation) writes out fused operations.
 #define SMPC_REAL double
 #define SMPC_FAST_F32 0
 #define SMPC_COLLIDE_NT 128
 #define SMPC_COLLIDE_CT 64
 #define SMPC_COLLIDE_CAP 768
+#define SMPC_COLLIDE_BLOCKS 3
 #define SMPC_BIN_NT 256
 #define SMPC_MD_NT 256
 #define SMPC_MD_MPT 4

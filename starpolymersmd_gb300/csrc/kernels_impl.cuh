@@ -2,6 +2,7 @@
 // those defines SMPC_REAL and the tile constants and includes this file once.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include "launch.h"
 #include "md_kernels.cuh"
 #if SMPC_FAST_F32
@@ -17,8 +18,12 @@ namespace smpc {
 typedef SMPC_REAL Real;
 
 template <>
-int collide_cells_per_tile<Real>() {
-  return SMPC_COLLIDE_CT;
+int collide_cells_per_tile<Real>(double density) {
+  // few enough that nearly every tile's particles (3.5 deviations) fit the
+  // staging; what does not is read again from global memory in each pass
+  int n = SMPC_COLLIDE_CT;
+  while (n > 1 && n * density + 3.5 * std::sqrt(n * density) > SMPC_COLLIDE_CAP) --n;
+  return n > 32 ? n - n % 32 : n;  // whole warps draw for the cells
 }
 
 template <typename R>
@@ -111,11 +116,13 @@ void launch_collide<Real>(const CollideArgs<Real>& a, cudaStream_t st) {
     return;
   }
 #endif
-  auto kern = k_collide<Real, SMPC_COLLIDE_NT, SMPC_COLLIDE_CT, SMPC_COLLIDE_CAP>;
-  const size_t dyn = collide_dyn_smem<Real>(SMPC_COLLIDE_CAP);
+  auto kern = k_collide<Real, SMPC_COLLIDE_NT, SMPC_COLLIDE_CT, SMPC_COLLIDE_CAP,
+                        SMPC_COLLIDE_BLOCKS>;
+  const size_t dyn = collide_dyn_smem<Real>(SMPC_COLLIDE_CAP, SMPC_COLLIDE_CT, a.amc != 0);
+  constexpr size_t most = collide_dyn_smem<Real>(SMPC_COLLIDE_CAP, SMPC_COLLIDE_CT, true);
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(dyn));
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
     configured = true;
   }
   kern<<<a.n_tiles, SMPC_COLLIDE_NT, dyn, st>>>(

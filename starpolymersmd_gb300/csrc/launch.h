@@ -61,7 +61,7 @@ struct CollideArgs {
 
 // Tile geometry chosen per precision (register budget of k_collide).
 template <typename R>
-int collide_cells_per_tile();
+int collide_cells_per_tile(double density);  // of particles per cell
 int fluid_slots_per_tile(bool fp64, long long slots);
 int temperature_cells_per_tile();
 int md_max_monomers();

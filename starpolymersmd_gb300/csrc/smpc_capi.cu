@@ -1112,20 +1112,17 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
   }
   int rc = opt->precision == SMPC_FP64 ? create_buffers<double>(ctx) : create_buffers<float>(ctx);
   if (rc) return bail(rc, ctx->err);
-  const int ct = opt->precision == SMPC_FP64 ? smpc::collide_cells_per_tile<double>()
-                                             : smpc::collide_cells_per_tile<float>();
   std::vector<Tile> bin =
       make_tiles(ctx->reps, false, smpc::fluid_slots_per_tile(opt->precision == SMPC_FP64, ctx->total_slots));
   std::vector<Tile> col;
-  if (fast_path(ctx)) {
-    for (const RepInfo& ri : ctx->reps) {
-      const int n = smpc::collide_tile_cells(static_cast<double>(ri.slot_cap) / ri.n_cell, cells);
-      for (int b = 0; b < ri.n_cell; b += n)
-        col.push_back(Tile{static_cast<int>(&ri - ctx->reps.data()), ri.cell_base + b,
-                           ri.cell_base + std::min(ri.n_cell, b + n), 0});
-    }
-  } else {
-    col = make_tiles(ctx->reps, true, ct);
+  for (const RepInfo& ri : ctx->reps) {
+    const double density = static_cast<double>(ri.slot_cap) / ri.n_cell;
+    const int n = fast_path(ctx) ? smpc::collide_tile_cells(density, cells)
+                  : opt->precision == SMPC_FP64 ? smpc::collide_cells_per_tile<double>(density)
+                                                : smpc::collide_cells_per_tile<float>(density);
+    for (int b = 0; b < ri.n_cell; b += n)
+      col.push_back(Tile{static_cast<int>(&ri - ctx->reps.data()), ri.cell_base + b,
+                         ri.cell_base + std::min(ri.n_cell, b + n), 0});
   }
   ctx->h_tmp_tiles = make_tiles(ctx->reps, true, smpc::temperature_cells_per_tile());
   ctx->n_bin_tiles = static_cast<int>(bin.size());
