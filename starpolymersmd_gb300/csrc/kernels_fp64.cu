@@ -14,15 +14,16 @@
 
 namespace smpc {
 // Solvent slots per binning tile (one CTA): FP64 blocks hold two records per
-// thread in flight (k_fluid_bin), FP32 blocks four; up to 4,096 (FP64: 2,048), and down
-// to one round of a CTA's loads so that a small box still gives every SM four
-// CTAs to hide the atomics' round trips. One box of 80,000 particles: 79 tiles
-// of 1,024 bin in 6.4 us, 20 of 4,096 in 15; 1.5 M particles: 742 of 2,048 in
-// 18.0, 371 of 4,096 in 19.4.
+// thread in flight (k_fluid_bin), FP32 blocks four. At most two (four) rounds of
+// these, and down to one so that a small box still gives every SM several CTAs
+// to hide the atomics' round trips: FP32, 80,000 particles: 79 tiles of 1,024
+// bin in 6.4 us, 20 of 4,096 in 15; 1.5 M: 742 of 2,048 in 18.0, 371 of 4,096 in
+// 19.4. FP64, 640,000 particles: tiles of 512 in 49 us, of 1,024 and 2,048 in 54;
+// 1.25 M: 83, 83, 87.
 int fluid_slots_per_tile(bool fp64, long long slots) {
-  int n = fp64 ? 2048 : 4096;
+  int n = fp64 ? 1024 : 4096;
   const int least = fp64 ? 512 : 1024;
-  while (n > least && slots < n * 4ll * 152) n /= 2;
+  while (n > least && slots < n * (fp64 ? 8ll : 4ll) * 152) n /= 2;
   return n;
 }
 int temperature_cells_per_tile() { return 512; }

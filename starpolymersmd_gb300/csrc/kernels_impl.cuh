@@ -18,6 +18,11 @@ namespace smpc {
 typedef SMPC_REAL Real;
 
 template <>
+size_t geo_bytes<Real>() {
+  return sizeof(Geo<Real>);
+}
+
+template <>
 int collide_cells_per_tile<Real>(double density) {
   // few enough that nearly every tile's particles (3.5 deviations) fit the
   // staging; what does not is read again from global memory in each pass
@@ -53,7 +58,7 @@ template <>
 void launch_mono_prep<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, Real* mpos, Real* mvel,
                             uint2* mkey, int* mimg, uint32_t* count, ErrorState* err,
                             int mono_bin, int strict, FrameF* frames, double rot_c, double rot_s,
-                            int chunks, int n_adv, double adv_scale, int gen_shift,
+                            int chunks, int n_adv, double adv_scale, int gen_shift, void* geo,
                             cudaStream_t st) {
   // CTAs of one replica must not race on its delrx: k_cycle_begin first
   if (chunks > 1 && (n_adv > 0 || gen_shift)) {
@@ -63,7 +68,7 @@ void launch_mono_prep<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, Real* m
   const dim3 grid(n_rep, chunks > 0 ? chunks : 1);
   k_mono_prep<Real, 512><<<grid, 512, 0, st>>>(reps, dyn, mpos, mvel, mkey, mimg, count, err,
                                                mono_bin, strict, frames, rot_c, rot_s, n_adv,
-                                               adv_scale, gen_shift);
+                                               adv_scale, gen_shift, static_cast<Geo<Real>*>(geo));
 }
 
 #if SMPC_FAST_F32
@@ -84,7 +89,7 @@ template <>
 void launch_fluid_bin<Real>(const Tile* tiles, int n_tiles, const RepInfo* reps,
                             const RepDyn* dyn, const FrameF* frames, const Real* rec, uint2* keys,
                             uint32_t* count, ErrorState* err, int strict, int variant,
-                            int packed, Real* frame, cudaStream_t st) {
+                            int packed, Real* frame, const void* geo, cudaStream_t st) {
   if (n_tiles == 0) return;
 #if SMPC_FAST_F32
   if (!strict && variant >= 0) {  // variant < 0: the generic kernel (what k_collide recomputes)
@@ -101,8 +106,8 @@ void launch_fluid_bin<Real>(const Tile* tiles, int n_tiles, const RepInfo* reps,
 #endif
   (void)frames;
   (void)variant;
-  k_fluid_bin<Real, SMPC_BIN_NT><<<n_tiles, SMPC_BIN_NT, 0, st>>>(tiles, reps, dyn, rec, keys,
-                                                                  count, err, strict, frame);
+  k_fluid_bin<Real, SMPC_BIN_NT><<<n_tiles, SMPC_BIN_NT, 0, st>>>(
+      tiles, reps, dyn, rec, keys, count, err, strict, frame, static_cast<const Geo<Real>*>(geo));
 }
 
 template <>
@@ -127,8 +132,8 @@ void launch_collide<Real>(const CollideArgs<Real>& a, cudaStream_t st) {
   }
   kern<<<a.n_tiles, SMPC_COLLIDE_NT, dyn, st>>>(
       a.tiles, a.reps, a.dyn, a.off, a.perm, a.st_in, a.st_out, a.mpos, a.mvel, a.mkey, a.mimg,
-      a.inj_gamma, a.inj_uphi, a.inj_utheta, a.rng, a.rot_c, a.rot_s, a.strict, a.mono_bin, a.amc,
-      a.err, a.frame);
+      a.inj_gamma, a.inj_uphi, a.inj_utheta, a.rng, a.rot_c, a.rot_s, a.strict, a.amc, a.err, a.frame,
+      static_cast<const Geo<Real>*>(a.geo));
 }
 
 template <>

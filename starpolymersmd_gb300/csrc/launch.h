@@ -57,8 +57,13 @@ struct CollideArgs {
   // collision-frame records written by the binning just before (generic
   // kernel; FP64 contexts), or null: the collide recomputes them from st_in
   const R* frame;
+  const void* geo;  // written by launch_mono_prep
 };
 
+// Bytes of a replica's box geometry in the generic kernels (written by
+// launch_mono_prep for the binning and the collide).
+template <typename R>
+size_t geo_bytes();
 // Tile geometry chosen per precision (register budget of k_collide).
 template <typename R>
 int collide_cells_per_tile(double density);  // of particles per cell
@@ -77,12 +82,12 @@ template <typename R>
 void launch_mono_prep(const RepInfo* reps, RepDyn* dyn, int n_rep, R* mpos, R* mvel, uint2* mkey,
                       int* mimg, uint32_t* count, ErrorState* err, int mono_bin, int strict,
                       FrameF* frames, double rot_c, double rot_s, int chunks, int n_adv, double adv_scale,
-                      int gen_shift, cudaStream_t st);
+                      int gen_shift, void* geo, cudaStream_t st);
 template <typename R>
 void launch_fluid_bin(const Tile* tiles, int n_tiles, const RepInfo* reps, const RepDyn* dyn,
                       const FrameF* frames, const R* rec, uint2* keys, uint32_t* count,
                       ErrorState* err, int strict, int variant, int packed, R* frame,
-                      cudaStream_t st);
+                      const void* geo, cudaStream_t st);
 template <typename R>
 void launch_collide(const CollideArgs<R>& a, cudaStream_t st);
 template <typename R>

@@ -304,11 +304,23 @@ __device__ __forceinline__ void le_wrap(const Geo<float>& g, float& x, float& y,
 // aliasing included, range-checked only against the last cell like the
 // reference; otherwise every axis index is clamped into the box (the fast
 // path: positions exactly on the upper face round onto L in FP32).
+// x truncated to an integer. A conversion is one more instruction on the narrow
+// FP64 pipe, so for 0 <= x < 2^20 the integer is taken from the high word's
+// bits; the rest converts.
+__device__ __forceinline__ int trunc_int(float x) { return static_cast<int>(x); }
+static __device__ __noinline__ int trunc_int_general(double x) { return static_cast<int>(x); }
+__device__ __forceinline__ int trunc_int(double x) {
+  const int hi = __double2hiint(x);
+  if (static_cast<unsigned>(hi) >= 0x41300000u) return trunc_int_general(x);  // 2^20 up, negative, NaN
+  const int e = (hi >> 20) - 1023;
+  return e < 0 ? 0 : ((hi & 0xFFFFF) | 0x100000) >> (20 - e);
+}
+
 template <typename R>
 __device__ __forceinline__ uint32_t cell_of(const Geo<R>& g, R x, R y, R z, bool strict) {
-  int ix = static_cast<int>(r_add(x, g.half[0]));
-  int iy = static_cast<int>(r_add(y, g.half[1]));
-  int iz = static_cast<int>(r_add(z, g.half[2]));
+  int ix = trunc_int(r_add(x, g.half[0]));
+  int iy = trunc_int(r_add(y, g.half[1]));
+  int iz = trunc_int(r_add(z, g.half[2]));
   if (strict) {
     const int c = ix + g.Li[0] * iy + g.Li[0] * g.Li[1] * iz;
     return static_cast<uint32_t>(c);
@@ -551,7 +563,7 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
                                                   uint32_t* count, ErrorState* err,
                                                   int mono_bin, int strict, FrameF* frames,
                                                   double rot_c, double rot_s, int n_adv,
-                                                  double adv_scale, int gen_shift) {
+                                                  double adv_scale, int gen_shift, Geo<R>* geo) {
   static_assert(NT >= 192, "six warps sum the recentring");
   const int r = blockIdx.x;
   const RepInfo& ri = reps[r];
@@ -637,6 +649,7 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
   if (tid == 0) {
     if (blockIdx.y == 0) dn.recentre = out;
     s_geo = make_geo<R>(ri, now, mono_bin);
+    if (blockIdx.y == 0) geo[r] = s_geo;
   }
   __syncthreads();
   const Geo<R>& g = s_geo;
@@ -731,18 +744,16 @@ template <typename R, int NT>
 __global__ void __launch_bounds__(NT) k_fluid_bin(const Tile* tiles, const RepInfo* reps,
                                                   const RepDyn* dyn, const R* __restrict__ st,
                                                   uint2* __restrict__ keys, uint32_t* count,
-                                                  ErrorState* err, int strict, R* frame) {
+                                                  ErrorState* err, int strict, R* frame,
+                                                  const Geo<R>* geo) {
   // FP64: two records in flight per thread, so that two blocks fit per SM
   // (the FP64 work is latency-bound on the narrow pipe; more warps hide it)
   constexpr int U = std::is_same<R, double>::value ? 2 : 4;
   const Tile t = tiles[blockIdx.x];
   const RepInfo& ri = reps[t.rep];
-  // one thread's FP64 arithmetic and conversions (a tenth of the FP64 kernel
-  // when every thread repeated them)
-  __shared__ Geo<R> s_geo;
-  if (threadIdx.x == 0) s_geo = make_geo<R>(ri, dyn[t.rep], 0);
-  __syncthreads();
-  const Geo<R> g = s_geo;
+  // made by k_mono_prep: the FP64 arithmetic and conversions in every thread
+  // were a tenth of the FP64 kernel
+  const Geo<R> g = geo[t.rep];
   const uint32_t cbase = static_cast<uint32_t>(ri.cell_base);
   const uint32_t ncell = static_cast<uint32_t>(ri.n_cell);
   const unsigned lane = threadIdx.x & 31u;
@@ -856,7 +867,6 @@ struct CollideCtx {
   const uint2* mkey;
   const int* mimg;
   Geo<R> g;
-  RepDyn dn;
   R solvent_mass;
   uint32_t cbase;
   uint32_t c0;
@@ -1209,7 +1219,7 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_collide(
     const uint32_t* __restrict__ perm, const R* __restrict__ st_in, R* __restrict__ st_out,
     const R* mpos, R* mvel, const uint2* mkey, const int* mimg, const double* inj_gamma,
     const double* inj_uphi, const double* inj_utheta, int rng, double rot_c, double rot_s,
-    int strict, int mono_bin, int amc, ErrorState* err, const R* frame) {
+    int strict, int amc, ErrorState* err, const R* frame, const Geo<R>* geo) {
   constexpr int GU = 4;
   constexpr bool kFP64 = std::is_same<R, double>::value;
   typedef typename AccT<R>::type Acc;
@@ -1235,9 +1245,8 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_collide(
   C.mvel = mvel;
   C.mkey = mkey;
   C.mimg = mimg;
-  __shared__ Geo<R> s_geo;
-  if (threadIdx.x == 0) s_geo = make_geo<R>(ri, dyn[t.rep], mono_bin);
-  C.dn = dyn[t.rep];
+  C.g = geo[t.rep];
+  const unsigned long long step = dyn[t.rep].step;
   C.solvent_mass = static_cast<R>(ri.solvent_mass);
   C.cbase = static_cast<uint32_t>(ri.cell_base);
   C.c0 = static_cast<uint32_t>(t.begin);
@@ -1251,7 +1260,6 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_collide(
 
   for (int i = threadIdx.x; i <= nc; i += NT) s_off[i] = off[t.begin + i];
   __syncthreads();
-  C.g = s_geo;
   const uint32_t p0 = s_off[0], p1 = s_off[nc];
   const int n = static_cast<int>(p1 - p0);
   const int nloc = n < CAP ? n : CAP;
@@ -1402,8 +1410,8 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_collide(
         const uint32_t nnc = s_off[c + 1] - s_off[c];
         double Mc[9];
         const double sc = cell_scale<double>(nnc, s_scale[c], cgc, cgc - C.cbase, rng, inj_gamma,
-                                             ri.seed, C.dn.step, kT, err);
-        cell_rotation_scaled(cgc, cgc - C.cbase, rng, inj_uphi, inj_utheta, ri.seed, C.dn.step, rc,
+                                             ri.seed, step, kT, err);
+        cell_rotation_scaled(cgc, cgc - C.cbase, rng, inj_uphi, inj_utheta, ri.seed, step, rc,
                              rs, sc >= 0.0 ? sc : 1.0, Mc);
 #pragma unroll
         for (int q = 0; q < 9; ++q) s_rot[9 * c + q] = static_cast<R>(Mc[q]);
@@ -1412,9 +1420,9 @@ __global__ void __launch_bounds__(NT, BLOCKS) k_collide(
       goto apply;
     }
     if (half == 0) {
-      if (live) scale = cell_scale<R>(nn, ekin, cg, cl, rng, inj_gamma, ri.seed, C.dn.step, kT, err);
+      if (live) scale = cell_scale<R>(nn, ekin, cg, cl, rng, inj_gamma, ri.seed, step, kT, err);
     } else if (live) {
-      cell_rotation<R>(cg, cl, rng, inj_uphi, inj_utheta, ri.seed, C.dn.step, rc, rs, M);
+      cell_rotation<R>(cg, cl, rng, inj_uphi, inj_utheta, ri.seed, step, rc, rs, M);
     }
     {  // both lanes get lane 0's factor
       const R other = __shfl_xor_sync(0xFFFFFFFFu, scale, 1);

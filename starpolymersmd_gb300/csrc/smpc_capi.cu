@@ -113,6 +113,7 @@ struct smpc_ctx {
   double* d_inj = nullptr;  // gamma | u_phi | u_theta, total_cells each
   ErrorState* d_err = nullptr;
   smpc::FrameF* d_frames = nullptr;
+  unsigned char* d_geo = nullptr;  // geo_bytes per replica
   // molecules per replica (local monomer offsets) and their device tables
   std::vector<std::vector<int>> mol_start;
   int2* d_rep_mols = nullptr;  // per replica: first molecule, count
@@ -224,7 +225,7 @@ void launch_prep(smpc_ctx* ctx, int n_adv, double adv, int gen_shift) {
                             static_cast<R*>(ctx->d_mvel), ctx->d_mkey, ctx->d_mimg, ctx->d_count,
                             ctx->d_err, ctx->opt.mono_bin, ctx->opt.strict_cells, ctx->d_frames,
                             ctx->rot_c, ctx->rot_s, ctx->mono_chunks, n_adv, adv, gen_shift,
-                            ctx->st);
+                            ctx->d_geo, ctx->st);
 }
 
 // n_adv > 0: delrx is advanced by that many MD steps of adv h each (graph mode);
@@ -237,7 +238,8 @@ int launch_binning(smpc_ctx* ctx, int cur, int n_adv, double adv, int gen_shift)
   smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
                             ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
                             ctx->opt.angular_momentum ? -1 : ctx->var_bin,
-                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->st);
+                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo,
+                            ctx->st);
   ctx->frame_ok = ctx->d_frame != nullptr;
   smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
                     ctx->st);
@@ -279,6 +281,7 @@ smpc::CollideArgs<R> collide_args(smpc_ctx* ctx, int rng, int cur) {
   a.mono_bin = ctx->opt.mono_bin;
   a.amc = ctx->opt.angular_momentum ? 1 : 0;
   a.err = ctx->d_err;
+  a.geo = ctx->d_geo;
   a.frame = ctx->frame_ok ? static_cast<const R*>(ctx->d_frame) : nullptr;
   return a;
 }
@@ -340,7 +343,8 @@ int profiled_cycle(smpc_ctx* ctx, int cur, cudaEvent_t* ev) {
   smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
                             ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
                             ctx->opt.angular_momentum ? -1 : ctx->var_bin,
-                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->st);
+                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo,
+                            ctx->st);
   ctx->frame_ok = ctx->d_frame != nullptr;
   cudaEventRecord(ev[1 + PH_BIN], ctx->st);
   smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
@@ -764,7 +768,7 @@ void free_all(smpc_ctx* ctx) {
                   ctx->d_tpart, ctx->d_keys, ctx->d_perm, ctx->d_count, ctx->d_off, ctx->d_tsum,
                   ctx->d_mpos, ctx->d_mvel, ctx->d_mfrc, ctx->d_mver, ctx->d_mkey,
                   ctx->d_mimg, ctx->d_bond_start, ctx->d_bonds, ctx->d_nlist, ctx->d_ncount,
-                  ctx->d_md_order, ctx->d_inj, ctx->d_err, ctx->d_frames, ctx->d_rep_mols,
+                  ctx->d_md_order, ctx->d_inj, ctx->d_err, ctx->d_frames, ctx->d_geo, ctx->d_rep_mols,
                   ctx->d_mols, ctx->d_obs, ctx->d_prof, ctx->d_c6, ctx->d_dstage, ctx->d_mol_obs,
                   ctx->d_mol_rep, ctx->d_init_part};
   for (void* p : ptrs)
@@ -1133,7 +1137,10 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
             dalloc(&ctx->d_col_tiles, col.size()) == cudaSuccess &&
             dalloc(&ctx->d_tmp_tiles, ctx->h_tmp_tiles.size()) == cudaSuccess &&
             dalloc(&ctx->d_tpart, ctx->h_tmp_tiles.size()) == cudaSuccess &&
-            dalloc(&ctx->d_err, 1) == cudaSuccess && dalloc(&ctx->d_frames, n_rep) == cudaSuccess;
+            dalloc(&ctx->d_err, 1) == cudaSuccess && dalloc(&ctx->d_frames, n_rep) == cudaSuccess &&
+            dalloc(&ctx->d_geo, n_rep * (opt->precision == SMPC_FP64 ? smpc::geo_bytes<double>()
+                                                                     : smpc::geo_bytes<float>())) ==
+                cudaSuccess;
   if (!ok) return bail(SMPC_E_CUDA, "alloc");
   ok = cudaMemcpy(ctx->d_reps, ctx->reps.data(), n_rep * sizeof(RepInfo), cudaMemcpyHostToDevice) == cudaSuccess &&
        cudaMemcpy(ctx->d_dyn, ctx->dyn.data(), n_rep * sizeof(RepDyn), cudaMemcpyHostToDevice) == cudaSuccess &&
