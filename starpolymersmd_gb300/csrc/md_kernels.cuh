@@ -1530,7 +1530,15 @@ constexpr int MD_CLUSTER_CAP = 1024;
 constexpr int MDC_ECAP = 8192;  // flattened list entries of a CTA's beads
 constexpr int MDC_CCAP = 1024;  // candidate pairs per force batch
 constexpr int MDC_BCAP = 512;   // bonds of a CTA's beads
-constexpr float MDC_FAR = 4096.0f;
+constexpr int MDC_FAR_LOG2 = 12;
+constexpr float MDC_FAR = 1 << MDC_FAR_LOG2;
+
+// |x| >= MDC_FAR or not a number (FP64: from the high word, without an
+// instruction of the FP64 pipe; MDC_FAR is a power of two)
+__device__ __forceinline__ bool md_is_far(float x) { return !(fabsf(x) < MDC_FAR); }
+__device__ __forceinline__ bool md_is_far(double x) {
+  return (__double2hiint(x) & 0x7FFFFFFF) >= ((1023 + MDC_FAR_LOG2) << 20);
+}
 
 // Dynamic shared memory of k_md_cluster<R, NT, CS, KMAX> (byte offsets).
 template <typename R, int CS>
@@ -1574,6 +1582,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
   constexpr int NW = NT / 32;
   static_assert((NW & (NW - 1)) == 0, "a power of two of warps (candidate search)");
   constexpr bool kF64 = sizeof(R) == 8;
+  constexpr bool kBySum = kF64 && 3 * ((CAP + CS - 1) / CS) <= NT;  // a thread per force component
   using L = MdcLayout<R, CS>;
   __shared__ int s_wcnt[NW], s_woff[NW + 1];
   // per warp and round of 32 list entries: candidates before the round, and
@@ -1733,8 +1742,14 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
     v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
     f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
     xv[0] = pv.x; xv[1] = pv.y; xv[2] = pv.z;
-    for (int d = 0; d < 3; ++d) fk[d] = a.andersen ? f[d] * (dth / m) : (f[d] / m) * dth;
   }
+  // (dth / m and 1 / m once; the quotients have the division's bits)
+  const R c_andersen = dth / m, rm = kF64 ? R(1) / m : R(1);
+  auto increment = [&]() {
+    for (int d = 0; d < 3; ++d)
+      fk[d] = a.andersen ? f[d] * c_andersen : (kF64 ? div_exact(f[d], m, rm) : f[d] / m) * dth;
+  };
+  increment();
   cl.sync();  // every copy loaded before any CTA writes into another's
   if (!a.force_rebuild) flatten();  // (a forced rebuild flattens the new lists)
   int rebuilds = 0;
@@ -1762,8 +1777,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
           const R d0 = xk[0] - xv[0], d1 = xk[1] - xv[1], d2 = xk[2] - xv[2];
           over = r_sqrt((d0 * d0 + d1 * d1) + d2 * d2) > lim;
         }
-        const bool far = !(fabs(xk[0]) < R(MDC_FAR) && fabs(xk[1]) < R(MDC_FAR) &&
-                           fabs(xk[2]) < R(MDC_FAR));
+        const bool far = md_is_far(xk[0]) || md_is_far(xk[1]) || md_is_far(xk[2]);
         // this CTA's copy here; the other CTAs' below, by all threads
         sx[ik] = xk[0];
         sy[ik] = xk[1];
@@ -1838,6 +1852,94 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
     }
     if (rebuild) {
       ++rebuilds;
+      // Membership is d^2 <= r_v^2 in the state's precision; FP64 states decide it
+      // in FP32 outside a band of 2^-7 around r_v^2 (FP32 rounding of
+      // coordinates below MDC_FAR moves d^2 by far less) and in FP64 inside it.
+      const bool fast = kF64 && !far_now;
+      const float rv2_lo = static_cast<float>(rv2) * (1.0f - 0.0078125f);
+      const float rv2_hi = static_cast<float>(rv2) * (1.0f + 0.0078125f);
+      // list starts of the CTA's beads, from their lengths in s_cstart
+      auto list_starts = [&]() {
+        if (threadIdx.x < 32) {
+          int carry = 0;
+          for (int q0 = 0; q0 < own; q0 += 32) {
+            const int qq = q0 + static_cast<int>(threadIdx.x);
+            const int cnt = qq < own ? s_cstart[qq] : 0;
+            const int ci = md_warp_scan(cnt);
+            if (qq < own) s_lstart[qq] = carry + ci - cnt;
+            carry += __shfl_sync(0xFFFFFFFFu, ci, 31);
+          }
+          if (threadIdx.x == 0) {
+            s_lstart[own] = carry;
+            s_fits = carry <= MDC_ECAP;
+          }
+        }
+      };
+      if (kF64) {
+        // A CTA owns n / CS beads: testing each against all n, a warp 128 at a
+        // time, takes 15,000 cycles for 25 of 401 with everything around it;
+        // sorting all n into hash cells in every CTA and walking 27 of them
+        // per bead took 22,000. Counted first, then written, in ascending order.
+        const int lane = static_cast<int>(threadIdx.x & 31u), w = static_cast<int>(threadIdx.x >> 5);
+        // the ballots of a bead's tests, 32 at most, wait in the candidate buffer
+        static_assert(MDC_ECAP >= 32 * ((CAP + CS - 1) / CS), "room for the ballots");
+        for (int qq = w; qq < own; qq += NW) {
+          const int ii = rank + CS * qq;
+          const float xf0 = pxf[ii], xf1 = pyf[ii], xf2 = pzf[ii];
+          int cnt = 0;
+          constexpr int U = 4;  // loads and tests in flight
+          for (int j0 = 0; j0 < n; j0 += 32 * U) {
+            bool in[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const int j = j0 + 32 * u + lane, jc = min(j, n - 1);
+              const float e0 = pxf[jc] - xf0, e1 = pyf[jc] - xf1, e2 = pzf[jc] - xf2;
+              const float r2f = fmaf(e0, e0, fmaf(e1, e1, e2 * e2));
+              in[u] = r2f < rv2_lo;
+              if (!fast || !(in[u] || r2f > rv2_hi)) {
+                const R d0 = sx[jc] - sx[ii], d1 = sy[jc] - sy[ii], d2 = sz[jc] - sz[ii];
+                in[u] = (d0 * d0 + d1 * d1) + d2 * d2 <= rv2;
+              }
+              in[u] = in[u] && j < n && j != ii;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const unsigned mk = __ballot_sync(0xFFFFFFFFu, in[u]);
+              if (lane == 0 && j0 + 32 * u < n) s_cand[32 * qq + (j0 >> 5) + u] = static_cast<int>(mk);
+              cnt += __popc(mk);
+            }
+          }
+          if (lane == 0) {
+            if (cnt > a.max_nb) {
+              raise_error(a.err, ERR_NEIGHBOR_OVF, static_cast<uint32_t>(b + ii),
+                          static_cast<uint32_t>(cnt));
+              cnt = a.max_nb;
+            }
+            a.ncount[b + ii] = cnt;
+            s_cstart[qq] = cnt;
+          }
+        }
+        __syncthreads();
+        list_starts();
+        __syncthreads();
+        for (int qq = w; qq < own; qq += NW) {
+          const int ii = rank + CS * qq, first = s_lstart[qq];
+          int cnt = 0;
+#pragma unroll 4
+          for (int c = 0; c < (n + 31) >> 5; ++c) {
+            const unsigned mk = static_cast<unsigned>(s_cand[32 * qq + c]);
+            const int pos = cnt + __popc(mk & ((1u << lane) - 1u)), j = 32 * c + lane;
+            if ((mk >> lane & 1u) && pos < a.max_nb) {
+              a.nlist[static_cast<size_t>(pos) * a.n_mono_total + b + ii] = b + j;
+              if (s_fits) {
+                s_nb[first + pos] = static_cast<unsigned short>(j);
+                s_own[first + pos] = static_cast<unsigned char>(qq);
+              }
+            }
+            cnt += __popc(mk);
+          }
+        }
+      } else {
       const R inv_rv = R(1) / static_cast<R>(ri.r_verlet);
       for (int j = threadIdx.x; j < n; j += NT) {
         const int cx = static_cast<int>(floor(sx[j] * inv_rv));
@@ -1850,14 +1952,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       md_bucket_sort<NT>(n, s_next, s_head, s_sorted);
       // Lists: the lanes of a bead split its 27 cells (cell t to lane t mod
       // lanes), count their members, then write them at the offsets the
-      // counts give, so a list holds lane 0's cells, then lane 1's, and so
-      // on. Membership is d^2 <= r_v^2 in the state's precision; FP64 states
-      // decide it in FP32 outside a band of 2^-7 around r_v^2 (FP32 rounding
-      // of coordinates below MDC_FAR moves d^2 by far less) and in FP64
-      // inside it.
-      const bool fast = kF64 && !far_now;
-      const float rv2_lo = static_cast<float>(rv2) * (1.0f - 0.0078125f);
-      const float rv2_hi = static_cast<float>(rv2) * (1.0f + 0.0078125f);
+      // counts give, so a list holds lane 0's cells, then lane 1's, and so on.
       int ccx = 0, ccy = 0, ccz = 0;
       float xf0 = 0.f, xf1 = 0.f, xf2 = 0.f;
       if (mine) {
@@ -1935,20 +2030,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         s_cstart[q] = cnt;
       }
       const int spill = __syncthreads_or(mc > MDC_SCRATCH);
-      if (threadIdx.x < 32) {  // list starts of the CTA's beads
-        int carry = 0;
-        for (int q0 = 0; q0 < own; q0 += 32) {
-          const int qq = q0 + static_cast<int>(threadIdx.x);
-          const int cnt = qq < own ? s_cstart[qq] : 0;
-          const int ci = md_warp_scan(cnt);
-          if (qq < own) s_lstart[qq] = carry + ci - cnt;
-          carry += __shfl_sync(0xFFFFFFFFu, ci, 31);
-        }
-        if (threadIdx.x == 0) {
-          s_lstart[own] = carry;
-          s_fits = carry <= MDC_ECAP;
-        }
-      }
+      list_starts();
       __syncthreads();
       if (mine) {
         int k = inc - mc;  // this lane's first list position
@@ -1967,6 +2049,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         } else {
           walk(put);
         }
+      }
       }
       if (kicker) { xv[0] = xk[0]; xv[1] = xk[1]; xv[2] = xk[2]; }
       for (int j = threadIdx.x; j < n; j += NT) {
@@ -2029,6 +2112,11 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         return s_woff[wq] + s_rpre[o >> 5][wq] + __popc(s_rmask[o >> 5][wq] & below);
       };
       R F0 = R(0), F1 = R(0), F2 = R(0);
+      // FP64: one thread per component of a bead's force adds all of it (in the
+      // bead's lanes, three components and a butterfly each, the additions took
+      // four times as many instructions of the narrow pipe); F0 and F1 are its
+      // even and odd terms
+      const int qs = static_cast<int>(threadIdx.x) / 3, ds = static_cast<int>(threadIdx.x) - 3 * qs;
       for (int c0 = 0; c0 == 0 || c0 < C; c0 += MDC_CCAP) {
         const int c1 = min(C, c0 + MDC_CCAP);
         // 2. FP64 pair forces of the candidates, then the bonds (first batch)
@@ -2075,7 +2163,17 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         __syncthreads();
         // 3. each bead's lanes: lane sub takes the bead's candidates
         // cs + sub, cs + sub + lanes, ... (cs its first)
-        if (mine) {
+        if (kBySum) {
+          if (qs < own) {
+            const int e1 = min(cand_before(s_lstart[qs + 1]), c1);
+            int c = max(cand_before(s_lstart[qs]), c0);
+            for (; c + 1 < e1; c += 2) {
+              F0 -= s_pf[3 * (c - c0) + ds];
+              F1 -= s_pf[3 * (c + 1 - c0) + ds];
+            }
+            if (c < e1) F0 -= s_pf[3 * (c - c0) + ds];
+          }
+        } else if (mine) {
           const int cs = cand_before(s_lstart[q]), e1 = min(cand_before(s_lstart[q + 1]), c1);
           const int st = max(cs, c0);
           for (int c = st + (((sub - (st - cs)) % nl) + nl) % nl; c < e1; c += nl) {
@@ -2087,6 +2185,12 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         }
         __syncthreads();  // read before the next batch rewrites the buffer
       }
+      if (kBySum) {
+        if (qs < own) {
+          for (int e = s_bstart[qs]; e < s_bstart[qs + 1]; ++e) F1 -= s_bf[3 * e + ds];
+          s_f[threadIdx.x] = F0 + F1;
+        }
+      } else {
       if (mine) {  // then its bonds, the same way
         for (int e = s_bstart[q] + sub; e < s_bstart[q + 1]; e += nl) {
           F0 -= s_bf[3 * e];
@@ -2103,6 +2207,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         s_f[3 * q] = F0;
         s_f[3 * q + 1] = F1;
         s_f[3 * q + 2] = F2;
+      }
       }
     } else {
     R F[3] = {R(0), R(0), R(0)};
@@ -2126,7 +2231,7 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       f[0] = s_f[3 * kq];
       f[1] = s_f[3 * kq + 1];
       f[2] = s_f[3 * kq + 2];
-      for (int d = 0; d < 3; ++d) fk[d] = a.andersen ? f[d] * (dth / m) : (f[d] / m) * dth;
+      increment();
       if (a.n_steps > 0) {
         for (int d = 0; d < 3; ++d)  // second half-kick
           v[d] += fk[d];
