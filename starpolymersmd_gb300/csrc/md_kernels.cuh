@@ -176,6 +176,27 @@ __device__ __forceinline__ void andersen_draw(unsigned long long seed, int bead,
   v[2] = s * (r2 * c2);
 }
 
+// One half of the same draw in FP64, so that two threads share its latency:
+// components 0 and 1 (half 0) or 2 of the bead's new velocity, sd = sqrt(kT / m).
+// Whether there is one goes to *set.
+static __device__ __forceinline__ void andersen_half(unsigned long long seed, int bead,
+                                                     unsigned long long md_step, double p, double sd,
+                                                     int half, double* v, unsigned char* set) {
+  const uint32_t c = ANDERSEN_STREAM | static_cast<uint32_t>(bead);
+  const Uniform2<double> a = philox_uniforms<double>(seed, c, md_step, 0u);
+  const bool reset = a.a < p;
+  if (half == 0) *set = reset ? 1 : 0;
+  if (!reset) return;
+  const Uniform2<double> b = philox_uniforms<double>(seed, c, md_step, 1u);
+  double turn = b.a;
+  if (half != 0) turn = philox_uniforms<double>(seed, c, md_step, 2u).a;
+  const double radius = ::sqrt(-2.0 * ::log(half == 0 ? a.b : b.b));
+  double sn, cs;
+  ::sincospi(2.0 * turn, &sn, &cs);
+  v[half == 0 ? 0 : 2] = sd * (radius * cs);
+  if (half == 0) v[1] = sd * (radius * sn);
+}
+
 // FENE (Potentials.h:24-55): anchor bonds (core) use R0^2 = 20.25.
 template <typename R>
 __device__ __forceinline__ R fene_force(bool anchor, R r2) {
@@ -1750,6 +1771,24 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       fk[d] = a.andersen ? f[d] * c_andersen : (kF64 ? div_exact(f[d], m, rm) : f[d] / m) * dth;
   };
   increment();
+  // FP64 Andersen draws (not staged ones) depend on the counters only: the
+  // upper half of the block makes them beside the lower half's force sums,
+  // two threads per bead, instead of each kick thread after its force, where
+  // they were 4.5 of a substep's 17 us.
+  constexpr int HALF = NT / 2;
+  constexpr bool kDraw = kBySum && 2 * ((CAP + CS - 1) / CS) <= HALF;
+  __shared__ double s_vn[kDraw ? 3 * (HALF / 2) : 1];
+  __shared__ unsigned char s_vset[kDraw ? HALF / 2 : 1];
+  const int* const staged_at =
+      a.and_start ? a.and_start + static_cast<size_t>(r) * (a.n_steps + 1) : nullptr;
+  const bool draws = kDraw && a.andersen && a.n_steps > 0 && !(staged_at && staged_at[0] >= 0);
+  const int drawer = static_cast<int>(threadIdx.x) - HALF, draw_q = drawer & (HALF / 2 - 1);
+  const bool drawing = draws && drawer >= 0 && draw_q < own;
+  double draw_p = 0.0, draw_sd = 0.0;
+  if (drawing) {
+    draw_p = a.andersen_nu * ri.md_dt;
+    draw_sd = ::sqrt(ri.kT) / ::sqrt(static_cast<double>(ld4_rw(mpos, b + rank + CS * draw_q).w));
+  }
   cl.sync();  // every copy loaded before any CTA writes into another's
   if (!a.force_rebuild) flatten();  // (a forced rebuild flattens the new lists)
   int rebuilds = 0;
@@ -2226,6 +2265,9 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       s_f[3 * q + 2] = F2;
     }
     }
+    if (drawing)
+      andersen_half(ri.seed, rank + CS * draw_q, md_step0 + static_cast<unsigned long long>(step),
+                    draw_p, draw_sd, drawer / (HALF / 2), s_vn + 3 * draw_q, s_vset + draw_q);
     __syncthreads();  // the forces reach the kick threads
     if (kicker) {
       f[0] = s_f[3 * kq];
@@ -2235,7 +2277,12 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       if (a.n_steps > 0) {
         for (int d = 0; d < 3; ++d)  // second half-kick
           v[d] += fk[d];
-        if (a.andersen) md_andersen_reset<R>(a, ri, r, step, ik, md_step0, m, v);
+        if (draws) {
+          if (s_vset[kq])
+            for (int d = 0; d < 3; ++d) v[d] = static_cast<R>(s_vn[3 * kq + d]);
+        } else if (a.andersen) {
+          md_andersen_reset<R>(a, ri, r, step, ik, md_step0, m, v);
+        }
       }
     }
   }
