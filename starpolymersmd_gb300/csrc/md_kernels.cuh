@@ -1821,11 +1821,6 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         sx[ik] = xk[0];
         sy[ik] = xk[1];
         sz[ik] = xk[2];
-        if (kF64) {
-          pxf[ik] = static_cast<float>(xk[0]);
-          pyf[ik] = static_cast<float>(xk[1]);
-          pzf[ik] = static_cast<float>(xk[2]);
-        }
         if (over || far)
           for (int c = 0; c < CS; ++c) {
             if (over) *cl.map_shared_rank(&s_rebuild[cur], c) = 1;
@@ -1839,7 +1834,6 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       // buffers lie at fixed offsets in the dynamic shared memory).
       __syncthreads();
       const size_t ox = reinterpret_cast<const unsigned char*>(sx) - s_dyn;
-      const size_t of = reinterpret_cast<const unsigned char*>(pxf) - s_dyn;
       for (int t = threadIdx.x; t < own * (CS - 1); t += NT) {
         const int bq = t / (CS - 1);
         const int c0 = t - bq * (CS - 1);
@@ -1850,15 +1844,16 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
         rx[ib] = sx[ib];
         rx[CAP + ib] = sy[ib];
         rx[2 * CAP + ib] = sz[ib];
-        if (kF64) {
-          float* fx = reinterpret_cast<float*>(base + of);
-          fx[ib] = pxf[ib];
-          fx[CAP + ib] = pyf[ib];
-          fx[2 * CAP + ib] = pzf[ib];
-        }
       }
     }
     cl.sync();  // positions and flags of this substep complete in every CTA
+    // each CTA rounds for itself: half of what went between them was rounded copies
+    if (kF64 && a.n_steps > 0)
+      for (int j = threadIdx.x; j < n; j += NT) {
+        pxf[j] = static_cast<float>(sx[j]);
+        pyf[j] = static_cast<float>(sy[j]);
+        pzf[j] = static_cast<float>(sz[j]);
+      }
     if (mine) { x[0] = sx[i]; x[1] = sy[i]; x[2] = sz[i]; }
     const bool far_now = s_far || s_farp[cur];
     bool over_here = s_rebuild[cur] != 0;
@@ -1876,7 +1871,9 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       if (kF64 && far_now) {
         over_here = true;
       } else {
-        const float c0 = pxf[0] - s_coref[0], c1 = pyf[0] - s_coref[1], c2 = pzf[0] - s_coref[2];
+        const float c0 = static_cast<float>(sx[0]) - s_coref[0],
+                    c1 = static_cast<float>(sy[0]) - s_coref[1],
+                    c2 = static_cast<float>(sz[0]) - s_coref[2];
         for (int j = threadIdx.x; j < n; j += NT) {
           const float d0 = pxf[j] - s_xvf[j] - c0, d1 = pyf[j] - s_xvf[CAP + j] - c1,
                       d2 = pzf[j] - s_xvf[2 * CAP + j] - c2;
