@@ -58,9 +58,10 @@ template <>
 void launch_mono_prep<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, Real* mpos, Real* mvel,
                             uint2* mkey, int* mimg, uint32_t* count, ErrorState* err,
                             int mono_bin, int strict, FrameF* frames, double rot_c, double rot_s,
-                            int chunks, int n_adv, double adv_scale, int gen_shift, void* geo,
+                            int chunks, int n_adv, double adv_scale, int gen_shift, void* geo, int part,
                             cudaStream_t st) {
   // CTAs of one replica must not race on its delrx: k_cycle_begin first
+  if (part == PREP_FRAME) chunks = 1;
   if (chunks > 1 && (n_adv > 0 || gen_shift)) {
     launch_cycle_begin<Real>(reps, dyn, n_rep, n_adv, adv_scale, gen_shift, st);
     n_adv = gen_shift = 0;
@@ -68,7 +69,7 @@ void launch_mono_prep<Real>(const RepInfo* reps, RepDyn* dyn, int n_rep, Real* m
   const dim3 grid(n_rep, chunks > 0 ? chunks : 1);
   k_mono_prep<Real, 512><<<grid, 512, 0, st>>>(reps, dyn, mpos, mvel, mkey, mimg, count, err,
                                                mono_bin, strict, frames, rot_c, rot_s, n_adv,
-                                               adv_scale, gen_shift, static_cast<Geo<Real>*>(geo));
+                                               adv_scale, gen_shift, static_cast<Geo<Real>*>(geo), part);
 }
 
 #if SMPC_FAST_F32
@@ -212,7 +213,8 @@ void launch_mono_stress<Real>(const RepInfo* reps, const RepDyn* dyn, int n_rep,
 template <>
 void launch_pmd_call<Real>(const PmdArgs& a, const RepInfo* reps, RepDyn* dyn, Real* mpos,
                            Real* mnext, Real* mvel, Real* mfrc, Real* mdisp, int n,
-                           double adv_scale, int calc_epot, int variant, cudaStream_t st) {
+                           double adv_scale, int calc_epot, int variant, cudaEvent_t drifted,
+                           cudaStream_t st) {
   if (a.n == 0) return;
   const int nb = a.n_blocks;
 #if SMPC_FAST_F32
@@ -240,11 +242,18 @@ void launch_pmd_call<Real>(const PmdArgs& a, const RepInfo* reps, RepDyn* dyn, R
     return;
   }
   k_pmd_drift<Real><<<nb, PMD_NT, 0, st>>>(a, reps, dyn, mpos, mvel, mfrc, mdisp, 1, adv_scale, 1);
+  if (drifted) cudaEventRecord(drifted, st);
   // the kernels after the drift follow their predecessor programmatically
   // (pmd_wait_previous): their launch overlaps its last blocks
-  cudaLaunchAttribute pdl[1];
+  cudaLaunchAttribute pdl[2];
   pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   pdl[0].val.programmaticStreamSerializationAllowed = 1;
+  int least = 0, greatest = 0;
+  if (drifted) {  // ahead of what runs beside them: a substep is a chain of short launches
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    pdl[1].id = cudaLaunchAttributePriority;
+    pdl[1].val.priority = greatest;
+  }
   auto cfg = [&](int blocks) {
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(blocks);
@@ -252,7 +261,7 @@ void launch_pmd_call<Real>(const PmdArgs& a, const RepInfo* reps, RepDyn* dyn, R
     c.dynamicSmemBytes = 0;
     c.stream = st;
     c.attrs = pdl;
-    c.numAttrs = 1;
+    c.numAttrs = drifted ? 2 : 1;
     return c;
   };
   for (int k = 1; k <= n; ++k) {

@@ -82,7 +82,7 @@ template <typename R>
 void launch_mono_prep(const RepInfo* reps, RepDyn* dyn, int n_rep, R* mpos, R* mvel, uint2* mkey,
                       int* mimg, uint32_t* count, ErrorState* err, int mono_bin, int strict,
                       FrameF* frames, double rot_c, double rot_s, int chunks, int n_adv, double adv_scale,
-                      int gen_shift, void* geo, cudaStream_t st);
+                      int gen_shift, void* geo, int part, cudaStream_t st);
 template <typename R>
 void launch_fluid_bin(const Tile* tiles, int n_tiles, const RepInfo* reps, const RepDyn* dyn,
                       const FrameF* frames, const R* rec, uint2* keys, uint32_t* count,
@@ -119,7 +119,7 @@ void launch_md(const MdArgs& a, int n_rep, R* mpos, R* mvel, R* mfrc, R* mver, i
 template <typename R>
 void launch_pmd_call(const PmdArgs& a, const RepInfo* reps, RepDyn* dyn, R* mpos, R* mnext,
                      R* mvel, R* mfrc, R* mdisp, int n, double adv_scale, int calc_epot,
-                     int variant, cudaStream_t st);
+                     int variant, cudaEvent_t drifted, cudaStream_t st);
 int pmd_block_count(int n_beads);
 
 // Molecules of periodic boxes made whole (observables.cuh); other boxes copied.

@@ -557,13 +557,17 @@ __global__ void k_init_velocity_finish(const RepInfo* reps, int rep, R* st, cons
 // add 1/32 of the beads, where all warps of the block issued six butterflies
 // on the FP64 pipe. Together with k_cycle_begin 20 us before, 10.7 now (one star
 // of 121 beads that recentres).
+//
+// part: all of it, the frame alone (what the solvent's binning waits for, where
+// no replica can recentre) or the monomers alone, once it exists.
 template <typename R, int NT>
 __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* dyn, R* mpos,
                                                   R* mvel, uint2* mkey, int* mimg,
                                                   uint32_t* count, ErrorState* err,
                                                   int mono_bin, int strict, FrameF* frames,
                                                   double rot_c, double rot_s, int n_adv,
-                                                  double adv_scale, int gen_shift, Geo<R>* geo) {
+                                                  double adv_scale, int gen_shift, Geo<R>* geo,
+                                                  int part) {
   static_assert(NT >= 192, "six warps sum the recentring");
   const int r = blockIdx.x;
   const RepInfo& ri = reps[r];
@@ -598,7 +602,9 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
   }
   const int per = split ? (ri.n_mono + gridDim.y - 1) / gridDim.y : ri.n_mono;
   const int b = ri.mono_base + static_cast<int>(blockIdx.y) * per;
-  const int n = max(0, min(per, ri.n_mono - static_cast<int>(blockIdx.y) * per));
+  const int n = part == PREP_FRAME
+                    ? 0
+                    : max(0, min(per, ri.n_mono - static_cast<int>(blockIdx.y) * per));
   // MPC.cpp:166: any monomer with |x_d| >= L_d/2 - 0.5 triggers recentring
   int over = 0;
   for (int i = tid; i < n && !split; i += NT) {
@@ -647,9 +653,11 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
     }
   }
   if (tid == 0) {
-    if (blockIdx.y == 0) dn.recentre = out;
     s_geo = make_geo<R>(ri, now, mono_bin);
-    if (blockIdx.y == 0) geo[r] = s_geo;
+    if (blockIdx.y == 0 && part != PREP_MONOMERS) {
+      dn.recentre = out;
+      geo[r] = s_geo;
+    }
   }
   __syncthreads();
   const Geo<R>& g = s_geo;
@@ -693,7 +701,7 @@ __global__ void __launch_bounds__(NT) k_mono_prep(const RepInfo* reps, RepDyn* d
       mimg[b + i] = img;
     }
   }
-  if (frames != nullptr && tid == NT - 32 && blockIdx.y == 0) {
+  if (frames != nullptr && tid == NT - 32 && blockIdx.y == 0 && part != PREP_MONOMERS) {
     FrameF f;
     for (int d = 0; d < 3; ++d) {
       f.L[d] = static_cast<float>(ri.L[d]);

@@ -220,31 +220,42 @@ void launch_permutation(smpc_ctx* ctx) {
 }
 
 template <typename R>
-void launch_prep(smpc_ctx* ctx, int n_adv, double adv, int gen_shift) {
+void launch_prep(smpc_ctx* ctx, int n_adv, double adv, int gen_shift, int part, cudaStream_t st) {
   smpc::launch_mono_prep<R>(ctx->d_reps, ctx->d_dyn, ctx->n_rep, static_cast<R*>(ctx->d_mpos),
                             static_cast<R*>(ctx->d_mvel), ctx->d_mkey, ctx->d_mimg, ctx->d_count,
                             ctx->d_err, ctx->opt.mono_bin, ctx->opt.strict_cells, ctx->d_frames,
                             ctx->rot_c, ctx->rot_s, ctx->mono_chunks, n_adv, adv, gen_shift,
-                            ctx->d_geo, ctx->st);
+                            ctx->d_geo, part, st);
+}
+
+template <typename R>
+void launch_solvent_binning(smpc_ctx* ctx, int cur, cudaStream_t st) {
+  smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
+                            ctx->d_frames, static_cast<const R*>(ctx->d_rec[cur]), ctx->d_keys,
+                            ctx->d_count, ctx->d_err, ctx->opt.strict_cells,
+                            ctx->opt.angular_momentum ? -1 : ctx->var_bin,
+                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo, st);
+  ctx->frame_ok = ctx->d_frame != nullptr;
 }
 
 // n_adv > 0: delrx is advanced by that many MD steps of adv h each (graph mode);
 // gen_shift: the device draws the grid shift from this collision's counter
 template <typename R>
 int launch_binning(smpc_ctx* ctx, int cur, int n_adv, double adv, int gen_shift) {
-  const int strict = ctx->opt.strict_cells;
-  const R* rec_in = static_cast<const R*>(ctx->d_rec[cur]);
-  launch_prep<R>(ctx, n_adv, adv, gen_shift);
-  smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
-                            ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
-                            ctx->opt.angular_momentum ? -1 : ctx->var_bin,
-                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo,
-                            ctx->st);
-  ctx->frame_ok = ctx->d_frame != nullptr;
+  launch_prep<R>(ctx, n_adv, adv, gen_shift, smpc::PREP_ALL, ctx->st);
+  launch_solvent_binning<R>(ctx, cur, ctx->st);
   smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
                     ctx->st);
   launch_permutation(ctx);
   return SMPC_OK;
+}
+
+template <typename R>
+void launch_sort_and_collide(smpc_ctx* ctx, int rng, int cur) {
+  smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
+                    ctx->st);
+  launch_permutation(ctx);
+  smpc::launch_collide<R>(collide_args<R>(ctx, rng, cur), ctx->st);
 }
 
 template <typename R>
@@ -287,14 +298,15 @@ smpc::CollideArgs<R> collide_args(smpc_ctx* ctx, int rng, int cur) {
 }
 
 template <typename R>
-int launch_md_steps(smpc_ctx* ctx, int n, int calc_epot, int force_rebuild) {
+int launch_md_steps(smpc_ctx* ctx, int n, int calc_epot, int force_rebuild,
+                    cudaEvent_t drifted = nullptr) {
   if (ctx->total_mono == 0) return SMPC_OK;
   const double adv = ctx->opt.delrx_mode == SMPC_DELRX_PHYSICAL ? 1.0 / ctx->opt.step_update : 1.0;
   for (const smpc::PmdArgs& p : ctx->pmd)
     smpc::launch_pmd_call<R>(p, ctx->d_reps, ctx->d_dyn, static_cast<R*>(ctx->d_mpos),
                              static_cast<R*>(ctx->d_mnext), static_cast<R*>(ctx->d_mvel),
                              static_cast<R*>(ctx->d_mfrc), static_cast<R*>(ctx->d_mver), n, adv,
-                             calc_epot, ctx->var_pmd, ctx->st);
+                             calc_epot, ctx->var_pmd, drifted, ctx->st);
   if (!ctx->any_local_md) return SMPC_OK;
   smpc::MdArgs a;
   a.reps = ctx->d_reps;
@@ -331,21 +343,14 @@ enum { PH_MD = 0, PH_BEGIN, PH_MONO, PH_BIN, PH_SCAN, PH_PERM, PH_COLLIDE, PH_EN
 template <typename R>
 int profiled_cycle(smpc_ctx* ctx, int cur, cudaEvent_t* ev) {
   const int nsub = ctx->opt.step_update;
-  const int strict = ctx->opt.strict_cells;
   const double adv = ctx->opt.delrx_mode == SMPC_DELRX_PHYSICAL ? 1.0 / nsub : 1.0;
-  const R* rec_in = static_cast<const R*>(ctx->d_rec[cur]);
   cudaEventRecord(ev[0], ctx->st);
   launch_md_steps<R>(ctx, nsub, 0, 0);
   cudaEventRecord(ev[1 + PH_MD], ctx->st);
   cudaEventRecord(ev[1 + PH_BEGIN], ctx->st);  // the collision's begin is part of PH_MONO
-  launch_prep<R>(ctx, nsub, adv, 1);
+  launch_prep<R>(ctx, nsub, adv, 1, smpc::PREP_ALL, ctx->st);
   cudaEventRecord(ev[1 + PH_MONO], ctx->st);
-  smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
-                            ctx->d_frames, rec_in, ctx->d_keys, ctx->d_count, ctx->d_err, strict,
-                            ctx->opt.angular_momentum ? -1 : ctx->var_bin,
-                            ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo,
-                            ctx->st);
-  ctx->frame_ok = ctx->d_frame != nullptr;
+  launch_solvent_binning<R>(ctx, cur, ctx->st);
   cudaEventRecord(ev[1 + PH_BIN], ctx->st);
   smpc::launch_scan(ctx->d_count, ctx->d_off, ctx->d_tsum, static_cast<int>(ctx->total_cells),
                     ctx->st);
@@ -363,11 +368,27 @@ int profiled_cycle(smpc_ctx* ctx, int cur, cudaEvent_t* ev) {
 template <typename R>
 int record_cycle(smpc_ctx* ctx, int cur) {
   const int nsub = ctx->opt.step_update;
-  launch_md_steps<R>(ctx, nsub, 0, 0);
   double adv = 1.0;
   if (ctx->opt.delrx_mode == SMPC_DELRX_PHYSICAL) adv = 1.0 / nsub;
   // h is per replica; delrx advances by shear*Ly*h*adv per MD step
-  launch_collision<R>(ctx, smpc::RNG_PHILOX, cur, nsub, adv);
+  if (ctx->n_rep == 1 && ctx->pmd.size() == 1 && !ctx->any_local_md &&
+      ctx->reps[0].mol0_size == 0 && ctx->total_slots > 0) {
+    // One periodic box: it never recentres, so its solvent is binned on a second
+    // stream beside the MD substeps, which are chains of short launches (100^3
+    // cells, 64 stars: 433 us per cycle, one after the other 456). The first
+    // of them reads delrx before the frame advances it.
+    launch_md_steps<R>(ctx, nsub, 0, 0, ctx->md_split.fork);
+    cudaStreamWaitEvent(ctx->md_split.st2, ctx->md_split.fork, 0);
+    launch_prep<R>(ctx, nsub, adv, 1, smpc::PREP_FRAME, ctx->md_split.st2);
+    launch_solvent_binning<R>(ctx, cur, ctx->md_split.st2);
+    cudaEventRecord(ctx->md_split.join, ctx->md_split.st2);
+    cudaStreamWaitEvent(ctx->st, ctx->md_split.join, 0);
+    launch_prep<R>(ctx, 0, 0.0, 0, smpc::PREP_MONOMERS, ctx->st);
+    launch_sort_and_collide<R>(ctx, smpc::RNG_PHILOX, cur);
+  } else {
+    launch_md_steps<R>(ctx, nsub, 0, 0);
+    launch_collision<R>(ctx, smpc::RNG_PHILOX, cur, nsub, adv);
+  }
   smpc::launch_cycle_end<R>(ctx->d_dyn, ctx->n_rep, ctx->st);
   return SMPC_OK;
 }
@@ -1468,7 +1489,7 @@ int smpc_cycles(smpc_ctx* ctx, int n) {
       cudaError_t e = cudaStreamEndCapture(ctx->st, &g);
       if (rc) return rc;
       if (e != cudaSuccess) return fail(ctx, SMPC_E_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-      e = cudaGraphInstantiate(&ctx->graph[cur], g, 0);
+      e = cudaGraphInstantiate(&ctx->graph[cur], g, cudaGraphInstantiateFlagUseNodePriority);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return fail(ctx, SMPC_E_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
     }

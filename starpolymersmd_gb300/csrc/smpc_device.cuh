@@ -38,6 +38,7 @@ enum : uint32_t {
 enum : int { POT_REF4824 = 0, POT_LJ126 = 1 };
 enum : int { MONOBIN_REFERENCE = 0, MONOBIN_WRAPPED = 1 };
 enum : int { RNG_INJECT = 0, RNG_PHILOX = 1 };
+enum : int { PREP_ALL = 0, PREP_FRAME = 1, PREP_MONOMERS = 2 };  // k_mono_prep
 enum : int { REP_PERIODIC_MD = 1 };  // smpc.h SMPC_REPLICA_PERIODIC_MD
 
 // Static per-replica description (uploaded once).
