@@ -185,13 +185,14 @@ int smpc_mpc_collide(smpc_ctx* ctx, const smpc_inject* inj);
 int smpc_cycles(smpc_ctx* ctx, int n);
 
 /* Same cycles launched on the context stream with CUDA events around every
- * phase (phase_ms[8]: MD substeps, cycle begin, monomer prep, solvent bin,
- * scan, perm, collide, cycle end; summed over the n cycles) and the total
+ * phase (phase_ms[8]: MD substeps, cycle begin (part of the monomer prep, so
+ * nothing of its own), monomer prep, solvent bin, scan, perm, collide, cycle
+ * end; summed over the n cycles; one phase after the other) and the total
  * elapsed time from the first to the last event. */
 int smpc_cycles_profiled(smpc_ctx* ctx, int n, double* phase_ms, int n_phases, double* total_ms);
 /* Launch-shape variants of the FP32 fast-path kernels (solvent binning,
- * collide, MD substeps); index 0 is the default. Changing them re-captures
- * the cycle graph. FP64 contexts of few replicas run each replica's MD on a
+ * collide, MD substeps); index 0 is the default. The collide has one shape:
+ * its indices 0 to 11 all name it. Changing them re-captures the cycle graph. FP64 contexts of few replicas run each replica's MD on a
  * cluster of SMs; md = 1 keeps one CTA per replica there instead. */
 int smpc_set_variants(smpc_ctx* ctx, int bin, int collide, int md);
 int smpc_get_variants(const smpc_ctx* ctx, int* bin, int* collide, int* md);
