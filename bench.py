@@ -36,7 +36,7 @@ import numpy as np  # noqa: E402
 
 METRIC = "MPC particle-updates/s"
 UNIT = "particle-updates/s"
-PHASE_LAUNCHES = 10  # kernels per cycle: md, begin, mono_prep, fluid_bin, 3x scan, perm, collide, end
+PHASE_LAUNCHES = 8   # kernels per cycle: md, mono_prep, fluid_bin, 2x scan, perm, collide, end
 PMD_LAUNCHES = 2     # kernels per MD substep of a periodic box (nlist, forces), plus 2 per cycle
 REF_MAX_STEPS = 20   # timed cycles of the reference arm (each ~0.6 s for batched_256 on 16 cores)
 
@@ -376,8 +376,11 @@ def run_ours(args, world, rank, local, dist):
              "frac": round(cycle_alg_bytes / (ms / K / 1e3) / 1e9 / peak, 4),
              "alg_bytes_per_cycle": cycle_alg_bytes}
 
-    launches_per_cycle = (PHASE_LAUNCHES - 1 + PMD_LAUNCHES * W.N_SUB + 2
+    # one periodic box prepares its frame and its monomers in two launches
+    launches_per_cycle = (PHASE_LAUNCHES - 1 + PMD_LAUNCHES * W.N_SUB + 2 + 1
                           if args.workload in W.PERIODIC else PHASE_LAUNCHES)
+    if n_cells <= 8192:
+        launches_per_cycle -= 1  # the scan of few cells is one launch
     big = sum(1 for n in built.n_mono if n > 512)
     if ctx.get_variants()[2] == 3 and 0 < big < built.n_rep:
         launches_per_cycle += 1  # the side-by-side MD shape runs two MD kernels
