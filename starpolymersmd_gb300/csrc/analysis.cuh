@@ -224,14 +224,15 @@ __global__ void __launch_bounds__(ANA_NT)
     part[12 * (static_cast<size_t>(r) * gridDim.y + blockIdx.y) + threadIdx.x] = s_tot[threadIdx.x];
 }
 
-// A replica's partial sums, in order, into out[12 r].
+// A replica's partial sums into out[12 r]: a warp per component.
 template <typename R>  // R: the precision of the instantiating unit (one copy per unit)
 __global__ void k_stress_reduce(const double* part, int n_part, double* out) {
-  const int r = blockIdx.x, k = threadIdx.x;
-  if (k >= 12) return;
+  const int r = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double t = 0.0;
-  for (int q = 0; q < n_part; ++q) t += part[12 * (static_cast<size_t>(r) * n_part + q) + k];
-  out[12 * static_cast<size_t>(r) + k] = t;
+  for (int q = lane; q < n_part; q += 32)
+    t += part[12 * (static_cast<size_t>(r) * n_part + q) + k];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, o);
+  if (lane == 0) out[12 * static_cast<size_t>(r) + k] = t;
 }
 
 }  // namespace smpc

@@ -207,7 +207,7 @@ void launch_mono_stress<Real>(const RepInfo* reps, const RepDyn* dyn, int n_rep,
   k_mono_stress<Real><<<dim3(n_rep, n_part), ANA_NT, 0, st>>>(reps, dyn, mpos, mvel, nlist_t,
                                                               ncount, n_mono_total, rows, max_nb,
                                                               bond_start, bonds, part);
-  k_stress_reduce<Real><<<n_rep, 32, 0, st>>>(part, n_part, out);
+  k_stress_reduce<Real><<<n_rep, 12 * 32, 0, st>>>(part, n_part, out);
 }
 
 template <>
@@ -293,7 +293,7 @@ void launch_velocity_profile<Real>(const RepInfo* reps, const int2* rep_mols, co
     k_velocity_profile<Real><<<(slot_cap + per_block - 1) / per_block, PROF_NT, 0, st>>>(
         reps, rep, rec, delrx, width, kx0, nx, ky0, ny, c6, bins, n_copies);
   const int n = 3 * (nx + ny);
-  k_profile_reduce<Real><<<(n + 255) / 256, 256, 0, st>>>(bins, n, n_copies, out);
+  k_profile_reduce<Real><<<(n + 7) / 8, 256, 0, st>>>(bins, n, n_copies, out);
 }
 
 // Monomer state between the device's R4 records and x,y,z-interleaved double

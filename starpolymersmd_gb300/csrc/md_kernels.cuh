@@ -1515,9 +1515,9 @@ __global__ void __launch_bounds__(NT, NT == 512 && KMAX > 1 ? 2 : 1)
 // rebuild flag. The copies are double-buffered by substep parity, so one
 // cluster barrier per substep, after the drift, suffices (positions and
 // flags complete everywhere); with displacements measured relative to the
-// core, every CTA decides the rebuild for all beads itself. A rebuild hashes
-// all beads in every CTA's own grid; each CTA writes the lists of its own
-// beads. Forces, kicks and the Andersen resets are those of k_md_substeps
+// core, every CTA decides the rebuild for all beads itself. In a rebuild each
+// CTA writes the lists of its own beads: found through a hash grid of all beads
+// (FP32), or by testing them against all (FP64). Forces, kicks and the Andersen resets are those of k_md_substeps
 // for the owned beads. The barriers are hardware cluster barriers: every CTA
 // of a cluster runs at once, and every CTA reaches every barrier (no branch
 // around one). Lowe-Andersen stays on k_md_substeps.

@@ -547,14 +547,16 @@ __global__ void __launch_bounds__(PROF_NT)
   prof_flush(yo, by);
 }
 
-// The copies of the bins, in order, into out.
+// The copies of the bins into out: a warp per bin, whose lanes add every 32nd
+// copy (one thread per bin added 128 of them one after the other, 19 us).
 template <typename R>  // R: the precision of the instantiating unit (one copy per unit)
 __global__ void k_profile_reduce(const double* bins, int n, int n_copies, double* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= n) return;
   double t = 0.0;
-  for (int c = 0; c < n_copies; ++c) t += bins[static_cast<size_t>(c) * n + i];
-  out[i] = t;
+  for (int c = lane; c < n_copies; c += 32) t += bins[static_cast<size_t>(c) * n + i];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, o);
+  if (lane == 0) out[i] = t;
 }
 
 }  // namespace smpc
