@@ -2,6 +2,7 @@
 // those defines SMPC_REAL and the tile constants and includes this file once.
 #pragma once
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include "launch.h"
 #include "md_kernels.cuh"
@@ -16,6 +17,19 @@
 namespace smpc {
 
 typedef SMPC_REAL Real;
+
+// Opts a kernel in to its dynamic shared memory, once per device (done: the
+// kernel's own, a bit per device).
+template <typename K>
+static void allow_shared(K kernel, size_t bytes, std::atomic<unsigned long long>& done) {
+  int device = 0;
+  cudaGetDevice(&device);
+  const unsigned long long bit = 1ull << (device & 63);
+  if (done.load(std::memory_order_relaxed) & bit) return;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(bytes)) == cudaSuccess)
+    done.fetch_or(bit, std::memory_order_relaxed);
+}
 
 template <>
 size_t geo_bytes<Real>() {
@@ -126,11 +140,8 @@ void launch_collide<Real>(const CollideArgs<Real>& a, cudaStream_t st) {
                         SMPC_COLLIDE_BLOCKS>;
   const size_t dyn = collide_dyn_smem<Real>(SMPC_COLLIDE_CAP, SMPC_COLLIDE_CT, a.amc != 0);
   constexpr size_t most = collide_dyn_smem<Real>(SMPC_COLLIDE_CAP, SMPC_COLLIDE_CT, true);
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
-    configured = true;
-  }
+  static std::atomic<unsigned long long> done{0};
+  allow_shared(kern, most, done);
   kern<<<a.n_tiles, SMPC_COLLIDE_NT, dyn, st>>>(
       a.tiles, a.reps, a.dyn, a.off, a.perm, a.st_in, a.st_out, a.mpos, a.mvel, a.mkey, a.mimg,
       a.inj_gamma, a.inj_uphi, a.inj_utheta, a.rng, a.rot_c, a.rot_s, a.strict, a.amc, a.err, a.frame,
@@ -359,10 +370,8 @@ void launch_pack_monomers<Real>(const Real* mpos, const Real* mvel, const Real* 
 template <int CS>
 static size_t md_cluster_smem() {
   constexpr size_t bytes = MdcLayout<Real, CS>::bytes;
-  static const bool set = cudaFuncSetAttribute(k_md_cluster<Real, 256, CS, 8>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(bytes)) == cudaSuccess;
-  (void)set;
+  static std::atomic<unsigned long long> done{0};
+  allow_shared(k_md_cluster<Real, 256, CS, 8>, bytes, done);
   return bytes;
 }
 
@@ -426,10 +435,8 @@ static void md_fast(const MdArgs& a, int blocks, float* mpos, float* mvel, float
                     cudaStream_t st) {
   constexpr size_t bytes = sizeof(MdFastSmem<NT, ROWS>);
   static_assert(bytes + 1024 <= (NT == 512 && KMAX > 1 ? 113 : 227) * 1024, "shared memory");
-  static const bool set = cudaFuncSetAttribute(k_md_fast<NT, KMAX, ROWS, U>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(bytes)) == cudaSuccess;
-  (void)set;
+  static std::atomic<unsigned long long> done{0};
+  allow_shared(k_md_fast<NT, KMAX, ROWS, U>, bytes, done);
   k_md_fast<NT, KMAX, ROWS, U><<<blocks, NT, bytes, st>>>(a, mpos, mvel, mfrc, mver);
 }
 #endif
