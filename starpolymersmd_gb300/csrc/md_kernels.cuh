@@ -926,12 +926,13 @@ struct MdFastSmem {
   float core_ref[3];
 };
 // Squared distance at the list build up to which a pair is kept: its cut-off
-// plus the skin, which two beads use up together before a rebuild, and a
-// margin far above FP32 rounding.
+// plus what two beads move together before a rebuild, and a margin far above
+// FP32 rounding. Each may move |r_verlet - r_cut| / 2, whichever is larger
+// (the core-relative test compares squares).
 __device__ __forceinline__ float md_keep_r2(int pot, bool bb, float skin) {
   const float cut2 = pot == POT_REF4824 ? (bb ? 2.25f : 1.0594631f)
                                         : (bb ? 6.25f : 1.2599210498948732f);
-  const float r = sqrtf(cut2) + fmaxf(skin, 0.0f) + 1e-3f;
+  const float r = sqrtf(cut2) + fabsf(skin) + 1e-3f;
   return r * r;
 }
 

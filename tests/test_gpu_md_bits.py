@@ -1,0 +1,58 @@
+"""The FP32 substeps with lists in shared memory (launch shape 0) and those with the
+lists in global memory (shape 1), both with one lane per bead, give the same bits:
+the Verlet lists, their order and the order of every sum are the same, and the pairs
+that shape 0 leaves out of its own lists carry exactly zero force until the next
+rebuild."""
+import numpy as np
+import pytest
+
+from starpolymersmd_gb300 import capi, system, workloads as W
+
+pytestmark = pytest.mark.gpu
+
+# arms, beads per arm, solvophobic share, r_cut, r_verlet, potential, Andersen
+LJ, REF = capi.POT_LJ126, capi.POT_REF4824
+CASES = {
+    "121": (6, 20, 0.5, 2.5, 2.8, LJ, False),
+    "401": (10, 40, 0.5, 2.5, 2.8, LJ, True),
+    "513": (16, 32, 0.6, 2.5, 2.8, LJ, False),
+    "1024": (11, 93, 0.4, 2.5, 3.0, LJ, False),
+    "reference_potential": (8, 30, 0.5, 1.5, 2.0, REF, False),
+    "thin_skin": (6, 30, 0.5, 2.5, 2.55, LJ, False),
+    # r_verlet below r_cut: the displacement that asks for a rebuild is |r_verlet - r_cut| / 2
+    "repulsive_below_r_cut": (8, 40, 0.0, 2.5, 1.6, LJ, False),
+    "reference_below_r_cut": (8, 40, 0.0, 1.5, 1.1, REF, True),
+    "attracting_below_r_cut": (8, 40, 0.5, 4.0, 2.8, LJ, False),
+}
+
+
+def _run(case, shape, calls):
+    arms, n_arm, frac, r_cut, r_verlet, pot, andersen = CASES[case]
+    spec = system.ReplicaSpec(L=40, arms=arms, n_arm=n_arm, solvophobic_fraction=frac, shear=0.1, seed=71)
+    st = system.make_star(arms, n_arm, frac, spec.mono_mass, spec.kT, np.random.default_rng(371), bond=0.97)
+    desc = dict(W.replica_desc(spec, st), n_fluid=0, potential=pot, r_cut=r_cut, r_verlet=r_verlet)
+    kw = dict(md_thermostat=capi.MDTHERMO_ANDERSEN, andersen_nu=1.0) if andersen else {}
+    out = []
+    with capi.Context([desc], precision=capi.FP32, rng=capi.RNG_PHILOX, max_neighbors=512,
+                      step_update=W.N_SUB, strict_cells=0, **kw) as ctx:
+        ctx.set_variants(0, 0, shape)
+        ctx.set_monomers(0, st.pos, st.vel, np.zeros_like(st.pos), np.full(st.n, st.mass), st.amphi, st.anchor)
+        ctx.set_bonds(0, st.bond_src, st.bond_dst)
+        ctx.init_md()
+        out.append(ctx.get_monomers(0))
+        for n in calls:  # most calls begin with the lists of the one before
+            ctx.md_substeps(n)
+            out.append(ctx.get_monomers(0))
+        if pot == LJ:  # (the reference's FENE reports bonds that a random start overstretches)
+            ctx.raise_on_device_error()
+        return out, ctx.verlet_rebuilds(0)
+
+
+@pytest.mark.parametrize("case", list(CASES))
+def test_lists_in_shared_memory_give_the_same_bits(case):
+    calls = (1, 3, 1, 10, 25)
+    (got, rebuilds), (want, expected) = (_run(case, shape, calls) for shape in (0, 1))
+    assert rebuilds == expected
+    for g, w in zip(got, want):
+        for a, b in zip(g, w):
+            np.testing.assert_array_equal(a, b)
