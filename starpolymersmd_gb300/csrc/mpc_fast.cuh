@@ -669,7 +669,9 @@ __global__ void __launch_bounds__(COL_NT, 15) k_collide_tile(
       const float inv = mt > 0.f ? 1.0f / mt : 0.0f;
       const float q0 = fix32_to_f(px), q1 = fix32_to_f(py), q2 = fix32_to_f(pz);
       const float ekin = cell_ekin(fix32_to_f(e), q0, q1, q2, inv);
-      const float sc = nn >= 2u && ekin > 0.f ? sqrtf(s_g[lc] / ekin) : 1.0f;
+      // (an injected variate without a square root: no thermostat)
+      const float factor = nn >= 2u && ekin > 0.f ? sqrtf(s_g[lc] / ekin) : 1.0f;
+      const float sc = factor >= 0.0f ? factor : 1.0f;
 #pragma unroll
       for (int r = 0; r < 3; r += 2) {  // rows 0 and 2 on the even lane, 1 on the odd one
         const int row = r + half;
