@@ -641,7 +641,8 @@ __global__ void __launch_bounds__(COL_NT, 15) k_collide_tile(
       pz = fix32_join(zh, zl, terms);
       e = fix32_join(eh, el, terms);
     }
-    if (n > nloc) {  // past the staging capacity
+    uint32_t over = 0;  // largest term past the staging capacity
+    if (n > nloc) {
       const CellSums o = cell_overflow((j0 > nloc ? j0 : nloc) + half, j1, p0, st_in, mpos, mvel, mimg,
                                        perm, f, mono_bin);
       px += o.px;
@@ -650,11 +651,12 @@ __global__ void __launch_bounds__(COL_NT, 15) k_collide_tile(
       e += o.e;
       nsol += o.nsol;
       mmono += o.mmono;
-      top = max(top, o.top);
+      over = o.top;
     }
     const uint32_t cg = static_cast<uint32_t>(t.begin + lc);
-    if (top >= __float_as_uint(FIX32_LIMIT)) {
-      if (pure && n <= nloc) top = largest_term(s_v, j0 + half, jl, ms);
+    if (max(top, over) >= __float_as_uint(FIX32_LIMIT)) {
+      if (pure) top = largest_term(s_v, j0 + half, jl, ms);  // without the NaN among them
+      top = max(top, over);
       if (top >= __float_as_uint(FIX32_LIMIT)) raise_cold(err, ERR_FIXPOINT, cg, top);
     }
     px += __shfl_xor_sync(FULL, px, 1);

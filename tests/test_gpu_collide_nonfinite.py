@@ -35,3 +35,18 @@ def test_a_gamma_variate_without_a_square_root_leaves_the_cell_unscaled(bad):
     assert word == strict_word == 0
     # velocities below 8, some ten roundings of 2^-24 each and a factor up to 2
     np.testing.assert_allclose(v, want, rtol=0, atol=2e-5)
+
+
+# 0: every tile fits its staging; 300: the tile of the first cell does not (360), and
+# holds particles that are not a number among the staged ones
+@pytest.mark.parametrize("extra", [0, 300])
+def test_velocities_that_are_no_numbers_are_reported_as_such_only(extra):
+    rng = np.random.default_rng(1)
+    pos, vel = _fluid(rng, 10 * N_CELL)
+    pos = np.concatenate([pos, (-2.5 + 0.4 * (rng.random((extra, 3)) - 0.5)).astype(np.float32)])
+    vel = np.concatenate([vel, rng.normal(size=(extra, 3)).astype(np.float32)])
+    bad = np.arange(0, 2000, 50)
+    vel[bad] = np.nan
+    word, v = _collide(pos, vel, rng.gamma(13.5, 1.0, N_CELL), rng.random(N_CELL), rng.random(N_CELL))
+    assert word == 8  # not finite; no term outside the fixed-point range
+    assert np.isnan(v[bad]).all()
