@@ -5,7 +5,8 @@
 //
 // Scan: two launches over C cells: per-tile scan (count is re-zeroed for the
 // next collision while it is read), then the totals of the tiles before are
-// added; one launch of one CTA for few cells. off[C] receives the total.
+// added; one launch of one CTA for few cells, and one between the two that
+// scans the totals for very many. off[C] receives the total.
 #include <stdint.h>
 
 #include "launch.h"
@@ -77,7 +78,10 @@ __global__ void __launch_bounds__(NT) k_scan_tiles(uint32_t* __restrict__ count,
 // for itself, beside its loads of the offsets, instead of waiting for a launch
 // that scans them. (A single launch with decoupled look-back, each tile polling
 // its predecessors' totals, took 9.3 us for 62 tiles and 67 for 3,907; the two
-// launches take 6.4 and 24, three with one for the totals took 9 and 28.)
+// launches take 6.4 and 24, three with one for the totals took 9 and 28; for
+// very many tiles see SCAN_MANY.)
+// SCANNED: tile_sum holds the sums before each tile already (k_scan_totals).
+template <bool SCANNED>
 __global__ void __launch_bounds__(SCAN_NT) k_scan_add(uint32_t* __restrict__ off,
                                                       const uint32_t* __restrict__ tile_sum,
                                                       int n) {
@@ -91,21 +95,66 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_add(uint32_t* __restrict__ off
     v[u] = i < n ? off[i] : 0u;
   }
   uint32_t before = 0;
+  if (SCANNED) {
+    before = tile_sum[tile];
+  } else {
 #pragma unroll 4
-  for (int t = threadIdx.x; t < tile; t += SCAN_NT) before += tile_sum[t];
-  before = __reduce_add_sync(0xFFFFFFFFu, before);
-  if (lane == 0) warp_tot[w] = before;
-  __syncthreads();
-  before = 0;
+    for (int t = threadIdx.x; t < tile; t += SCAN_NT) before += tile_sum[t];
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    if (lane == 0) warp_tot[w] = before;
+    __syncthreads();
+    before = 0;
 #pragma unroll
-  for (int q = 0; q < SCAN_NT / 32; ++q) before += warp_tot[q];
+    for (int q = 0; q < SCAN_NT / 32; ++q) before += warp_tot[q];
+  }
 #pragma unroll
   for (int u = 0; u < SCAN_IPT; ++u) {
     const int i = base + u * SCAN_NT;
     if (i < n) off[i] = v[u] + before;
   }
-  if (tile == static_cast<int>(gridDim.x) - 1 && threadIdx.x == 0)
+  if (!SCANNED && tile == static_cast<int>(gridDim.x) - 1 && threadIdx.x == 0)
     off[n] = before + tile_sum[tile];
+}
+
+// The tiles' totals, scanned in place by one CTA; off[n] receives their sum.
+constexpr int SCAN_TOT_NT = 1024, SCAN_TOT_IPT = 8;
+__global__ void __launch_bounds__(SCAN_TOT_NT) k_scan_totals(uint32_t* __restrict__ tile_sum,
+                                                             int tiles, uint32_t* __restrict__ off,
+                                                             int n) {
+  __shared__ uint32_t warp_tot[SCAN_TOT_NT / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (int base = 0; base < tiles; base += SCAN_TOT_NT * SCAN_TOT_IPT) {
+    const int first = base + threadIdx.x * SCAN_TOT_IPT;
+    uint32_t c[SCAN_TOT_IPT], own = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_TOT_IPT; ++k) {
+      c[k] = first + k < tiles ? tile_sum[first + k] : 0u;
+      own += c[k];
+    }
+    uint32_t x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_tot[w] = x;
+    __syncthreads();
+    uint32_t run = carry + x - own;
+#pragma unroll
+    for (int q = 0; q < SCAN_TOT_NT / 32; ++q) {
+      const uint32_t t = warp_tot[q];
+      if (q < w) run += t;
+      carry += t;
+    }
+#pragma unroll
+    for (int k = 0; k < SCAN_TOT_IPT; ++k) {
+      if (first + k < tiles) tile_sum[first + k] = run;
+      run += c[k];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) off[n] = carry;
 }
 
 // perm[off[cell] + rank] = source. Each thread takes PERM_U entries a block
@@ -202,6 +251,11 @@ __global__ void __launch_bounds__(PERM_NT) k_build_perm_packed(
 // four times as many cells per thread it took 12 us for 29,791.
 constexpr int SCAN_ONE_NT = 1024, SCAN_ONE_IPT = 8;
 constexpr int SCAN_ONE = SCAN_ONE_NT * SCAN_ONE_IPT;
+// Above this many tiles (67 M cells) a third launch scans their totals: every
+// CTA's own sum over the tiles before it grows with their number. Two launches
+// against three: 56 and 61 us for 8,192 tiles, 214 and 214 for 31,250, 370 and
+// 301 for 44,494, 668 and 410 for 61,035.
+constexpr int SCAN_MANY = 32768;
 int scan_tile_count(int n_cells) { return (n_cells + SCAN_TILE - 1) / SCAN_TILE; }
 
 void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, int n_cells,
@@ -213,7 +267,12 @@ void launch_scan(uint32_t* count, uint32_t* off, uint32_t* tile_sum, int n_cells
   }
   const int tiles = scan_tile_count(n_cells);
   k_scan_tiles<SCAN_NT, SCAN_IPT><<<tiles, SCAN_NT, 0, st>>>(count, off, tile_sum, n_cells);
-  k_scan_add<<<tiles, SCAN_NT, 0, st>>>(off, tile_sum, n_cells);
+  if (tiles > SCAN_MANY) {
+    k_scan_totals<<<1, SCAN_TOT_NT, 0, st>>>(tile_sum, tiles, off, n_cells);
+    k_scan_add<true><<<tiles, SCAN_NT, 0, st>>>(off, tile_sum, n_cells);
+  } else {
+    k_scan_add<false><<<tiles, SCAN_NT, 0, st>>>(off, tile_sum, n_cells);
+  }
 }
 
 void launch_build_perm_packed(const Tile* tiles, int n_tiles, const RepInfo* reps,
