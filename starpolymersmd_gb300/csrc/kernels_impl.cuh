@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 #include "launch.h"
 #include "md_kernels.cuh"
 #if SMPC_FAST_F32
@@ -37,12 +38,25 @@ size_t geo_bytes<Real>() {
 }
 
 template <>
-int collide_cells_per_tile<Real>(double density) {
+int collide_cells_per_tile<Real>(double density, long long total_cells) {
   // few enough that nearly every tile's particles (3.5 deviations) fit the
   // staging; what does not is read again from global memory in each pass
   int n = SMPC_COLLIDE_CT;
   while (n > 1 && n * density + 3.5 * std::sqrt(n * density) > SMPC_COLLIDE_CAP) --n;
-  return n > 32 ? n - n % 32 : n;  // whole warps draw for the cells
+  if (n > 32) return n - n % 32;  // whole warps draw for the cells
+  // FP64, more than 21 particles per cell: so few cells leave most lanes idle in
+  // the cell sums and the draws, which costs more than reading particles again
+  // wherever all tiles would be resident at once (three per SM) with more of
+  // them: 27,000 cells at 100 particles 601 us with 6 cells per tile, 360 with
+  // 64; 8,000 at 400 2,364 with one and 846 with 18; 1,728 at 1,000 1,631 with
+  // one and 1,317 with 4. At 20 per cell 32 that fit take 200 us for 64,000
+  // cells, 64 take 217.
+  if (std::is_same<Real, double>::value && n < 32) {
+    const long long wave = 152 * SMPC_COLLIDE_BLOCKS;
+    const int w = static_cast<int>(std::min<long long>((total_cells + wave - 1) / wave, SMPC_COLLIDE_CT));
+    n = std::max(n, w > 32 ? SMPC_COLLIDE_CT : w);
+  }
+  return n;
 }
 
 template <typename R>

@@ -66,7 +66,7 @@ template <typename R>
 size_t geo_bytes();
 // Tile geometry chosen per precision (register budget of k_collide).
 template <typename R>
-int collide_cells_per_tile(double density);  // of particles per cell
+int collide_cells_per_tile(double density, long long total_cells);  // density: particles per cell
 int fluid_slots_per_tile(bool fp64, long long slots);
 int temperature_cells_per_tile();
 int md_max_monomers();

@@ -1143,8 +1143,8 @@ int smpc_create(const smpc_replica_desc* descs, int n_rep, const smpc_options* o
   for (const RepInfo& ri : ctx->reps) {
     const double density = static_cast<double>(ri.slot_cap) / ri.n_cell;
     const int n = fast_path(ctx) ? smpc::collide_tile_cells(density, cells)
-                  : opt->precision == SMPC_FP64 ? smpc::collide_cells_per_tile<double>(density)
-                                                : smpc::collide_cells_per_tile<float>(density);
+                  : opt->precision == SMPC_FP64 ? smpc::collide_cells_per_tile<double>(density, cells)
+                                                : smpc::collide_cells_per_tile<float>(density, cells);
     for (int b = 0; b < ri.n_cell; b += n)
       col.push_back(Tile{static_cast<int>(&ri - ctx->reps.data()), ri.cell_base + b,
                          ri.cell_base + std::min(ri.n_cell, b + n), 0});
