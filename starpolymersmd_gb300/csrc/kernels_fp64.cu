@@ -28,7 +28,21 @@ int fluid_slots_per_tile(bool fp64, long long slots) {
 }
 int temperature_cells_per_tile() { return 512; }
 int md_max_monomers() { return SMPC_MD_NT * SMPC_MD_MPT; }
-int profile_copies(size_t bins) { return bins <= 65536 ? PROF_COPIES : 1; }
+// Runs so long that the SMs keep 1,024 threads each, up to 16 slots: 5,120
+// slots 44 us the call with runs of one and 70 with 16, 1.25 M 121 to 127 with 4
+// or 8 and 125 to 133 with 16, 10 M 593 to 626 with 16 and 888 with one.
+// Copies of the bins where 300 or more particles meet in one (bins counts three
+// doubles for each, x and y): 80,000 particles and 2,001 bins per axis take 48 us
+// without copies and 62 with 128 of them, 201 bins 61 and 52; 1.25 M particles and
+// 5,001 bins 129 and 154, 501 bins 162 and 133. No more copies than blocks, and
+// none past 65,536 doubles.
+ProfilePlan profile_plan(int slots, size_t bins) {
+  int run = 1;
+  while (run < 16 && slots >= 2 * run * 152 * 1024) run *= 2;
+  const int blocks = (slots + PROF_NT * run - 1) / (PROF_NT * run);
+  const bool copies = bins <= 65536 && static_cast<size_t>(slots) >= 50 * bins;
+  return {copies ? std::max(1, std::min(128, blocks)) : 1, run};
+}
 int stress_parts(int n_mono) {
   return std::max(1, std::min(1024, (n_mono * STRESS_LANES + ANA_NT - 1) / ANA_NT));
 }

@@ -311,14 +311,16 @@ void launch_velocity_profile<Real>(const RepInfo* reps, const int2* rep_mols, co
                                    int rep, int slot_cap, const Real* rec, const Real* mpos,
                                    const Real* mvel, double delrx, double width, long long kx0,
                                    int nx, long long ky0, int ny, double* c6, double* out,
-                                   double* bins, int n_copies, cudaStream_t st) {
+                                   double* bins, const ProfilePlan& plan, cudaStream_t st) {
   k_profile_centre<Real><<<1, PROF_NT, 0, st>>>(rep_mols, mols, mpos, mvel, rep, c6);
-  constexpr int per_block = PROF_NT * PROF_RUN;
+  const int per_block = PROF_NT * plan.run;
   if (slot_cap > 0)
     k_velocity_profile<Real><<<(slot_cap + per_block - 1) / per_block, PROF_NT, 0, st>>>(
-        reps, rep, rec, delrx, width, kx0, nx, ky0, ny, c6, bins, n_copies);
+        reps, rep, rec, delrx, width, kx0, nx, ky0, ny, c6, plan.copies > 1 ? bins : out, plan.copies,
+        plan.run);
   const int n = 3 * (nx + ny);
-  k_profile_reduce<Real><<<(n + 7) / 8, 256, 0, st>>>(bins, n, n_copies, out);
+  if (plan.copies > 1)
+    k_profile_reduce<Real><<<(n + 7) / 8, 256, 0, st>>>(bins, n, plan.copies, out);
 }
 
 // Monomer state between the device's R4 records and x,y,z-interleaved double

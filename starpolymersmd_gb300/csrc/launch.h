@@ -135,13 +135,18 @@ template <typename R>
 void launch_mol_observables(const int2* rep_mols, const int2* mols, int n_rep, int n_mols,
                             const R* mpos, const R* mvel, double* mol_out, double* out,
                             cudaStream_t st);
+// How the velocity profile adds up: `copies` copies of the bins behind each
+// other (one: straight into the result), `run` consecutive slots per thread.
+struct ProfilePlan {
+  int copies, run;
+};
+ProfilePlan profile_plan(int slots, size_t bins);  // bins: doubles
 template <typename R>
 void launch_velocity_profile(const RepInfo* reps, const int2* rep_mols, const int2* mols, int rep,
                              int slot_cap, const R* rec, const R* mpos, const R* mvel,
                              double delrx, double width, long long kx0, int nx, long long ky0,
-                             int ny, double* c6, double* out, double* bins, int n_copies,
-                             cudaStream_t st);
-int profile_copies(size_t bins);  // copies of `bins` doubles that the profile's blocks add into
+                             int ny, double* c6, double* out, double* bins,
+                             const ProfilePlan& plan, cudaStream_t st);
 
 // Solvent analyses (analysis.cuh); part: per-block partial sums.
 template <typename R>

@@ -415,8 +415,6 @@ __global__ void __launch_bounds__(UNWRAP_NT)
 }
 
 constexpr int PROF_NT = 128;   // threads per block of the profile kernels
-constexpr int PROF_RUN = 16;   // consecutive slots per thread of k_velocity_profile
-constexpr int PROF_COPIES = 128;  // copies of the bins that the blocks add into
 
 template <typename R>
 __global__ void __launch_bounds__(PROF_NT) k_profile_centre(const int2* rep_mols, const int2* mols,
@@ -484,7 +482,7 @@ __device__ __forceinline__ void prof_add(ProfAcc& even, ProfAcc& odd, long long 
 
 // bins: x then y, 3 doubles per bin (sum v_x, sum v_y, count), n_copies copies
 // zeroed by the host; block b adds into copy b mod n_copies. Every thread
-// walks PROF_RUN consecutive slots. The solvent is in cell order after a
+// walks `run` consecutive slots (profile_plan). The solvent is in cell order after a
 // collision, so a run meets a few bins only, two neighbouring ones per axis at
 // a time; their sums stay in registers (one pair for even bins, one for odd)
 // and go out when the bin changes. One atomic per particle and sum onto the
@@ -495,10 +493,10 @@ template <typename R>
 __global__ void __launch_bounds__(PROF_NT)
     k_velocity_profile(const RepInfo* reps, int rep, const R* rec, double delrx, double width,
                        long long kx0, int nx, long long ky0, int ny, const double* c6,
-                       double* bins, int n_copies) {
+                       double* bins, int n_copies, int run) {
   const RepInfo& ri = reps[rep];
-  const int i0 = (blockIdx.x * PROF_NT + threadIdx.x) * PROF_RUN;
-  const int i1 = min(i0 + PROF_RUN, ri.slot_cap);
+  const int i0 = (blockIdx.x * PROF_NT + threadIdx.x) * run;
+  const int i1 = min(i0 + run, ri.slot_cap);
   double* bx = bins + static_cast<size_t>(blockIdx.x % n_copies) * 3 * static_cast<size_t>(nx + ny);
   double* by = bx + 3 * static_cast<size_t>(nx);
   const double c0 = c6[0], c1 = c6[1], cv0 = c6[3], cv1 = c6[4];

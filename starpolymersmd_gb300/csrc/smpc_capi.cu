@@ -1928,8 +1928,8 @@ void velocity_profile_t(smpc_ctx* ctx, int rep, double width, long long kx0, int
                                    ctx->reps[rep].slot_cap,
                                    static_cast<const R*>(ctx->d_rec[ctx->cur]), p, v,
                                    ctx->dyn[rep].delrx, width, kx0, n_x, ky0, n_y, ctx->d_c6,
-                                   ctx->d_prof, ctx->d_prof + nb, smpc::profile_copies(nb),
-                                   ctx->st);
+                                   ctx->d_prof, ctx->d_prof + nb,
+                                   smpc::profile_plan(ctx->reps[rep].slot_cap, nb), ctx->st);
 }
 }  // namespace
 
@@ -2010,8 +2010,10 @@ int smpc_velocity_profile(smpc_ctx* ctx, int rep, double width, double* x_out, i
     return fail(ctx, SMPC_E_ARG, "profile needs " + std::to_string(need_x) + " x bins and " +
                                      std::to_string(need_y) + " y bins");
   cudaSetDevice(ctx->device);
-  // the result, then the copies that the blocks add into
-  const size_t nb = 3 * static_cast<size_t>(n_x + n_y), nc = nb * smpc::profile_copies(nb);
+  // the result, then the copies that the blocks add into (one: the result itself)
+  const size_t nb = 3 * static_cast<size_t>(n_x + n_y);
+  const int copies = smpc::profile_plan(ctx->reps[rep].slot_cap, nb).copies;
+  const size_t nc = copies > 1 ? nb * copies : 0;
   if (nb + nc > ctx->prof_cap) {
     CU(cudaStreamSynchronize(ctx->st));
     if (ctx->d_prof) cudaFree(ctx->d_prof);
@@ -2020,7 +2022,8 @@ int smpc_velocity_profile(smpc_ctx* ctx, int rep, double width, double* x_out, i
     CU(dalloc(&ctx->d_prof, nb + nc));
     ctx->prof_cap = nb + nc;
   }
-  CU(cudaMemsetAsync(ctx->d_prof + nb, 0, nc * sizeof(double), ctx->st));
+  CU(cudaMemsetAsync(copies > 1 ? ctx->d_prof + nb : ctx->d_prof, 0, std::max(nb, nc) * sizeof(double),
+                     ctx->st));
   if (ctx->total_mono > 0 && !ctx->md_ready && !ctx->pmd.empty())
     return fail(ctx, SMPC_E_STATE, "smpc_init_md not called (bonds make periodic molecules whole)");
   if (ctx->opt.precision == SMPC_FP64)
