@@ -976,18 +976,32 @@ static __device__ __noinline__ void md_bead_forces_global(const MdArgs& a, int b
   const int cnt = a.ncount[b + i];
   const int* nl = a.nlist + b + i;
   const size_t stride = static_cast<size_t>(a.n_mono_total);
-  for (int q = sub; q < cnt; q += 1 << lk) {
-    const int j = nl[static_cast<size_t>(q) * stride] - b;
-    const float4 y = pos[j];
-    const float d0 = y.x - x[0], d1 = y.y - x[1], d2 = y.z - x[2];
-    const float r2 = (d0 * d0 + d1 * d1) + d2 * d2;
-    const bool bb = ai && amphi[j] != 0;
-    const float fa = pair_force<float>(pot, bb, r2, lambda);
-    F0 -= d0 * fa;
-    F1 -= d1 * fa;
-    F2 -= d2 * fa;
-    if (want_epot) *epot += md_pair_epot<float>(pot, bb, r2, lambda);
+  constexpr int PF = 4;  // list loads in flight (8 cost the caller registers)
+  double ep = 0.0;
+#pragma unroll 1
+  for (int q0 = sub; q0 < cnt; q0 += PF << lk) {
+    int js[PF];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int q = q0 + (u << lk);
+      js[u] = q < cnt ? nl[static_cast<size_t>(q) * stride] - b : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < PF; ++u) {
+      const int j = js[u];
+      if (j < 0) break;
+      const float4 y = pos[j];
+      const float d0 = y.x - x[0], d1 = y.y - x[1], d2 = y.z - x[2];
+      const float r2 = (d0 * d0 + d1 * d1) + d2 * d2;
+      const bool bb = ai && amphi[j] != 0;
+      const float fa = pair_force<float>(pot, bb, r2, lambda);
+      F0 -= d0 * fa;
+      F1 -= d1 * fa;
+      F2 -= d2 * fa;
+      if (want_epot) ep += 0.5 * static_cast<double>(pair_pot<float>(pot, bb, r2, lambda));
+    }
   }
+  *epot += ep;
   if (sub == 0)
     for (int e = a.bond_start[b + i]; e < a.bond_start[b + i + 1]; ++e) {
       const int2 bd = a.bonds[e];
@@ -1391,7 +1405,9 @@ __global__ void __launch_bounds__(NT, NT == 512 && KMAX > 1 ? 2 : 1)
       S.bond[e] = static_cast<unsigned short>((bd.x - b) | (bd.y != 0 ? 0x8000 : 0));
     }
   }
-  int n_ent = -1;        // entries of this thread (-1: to be taken from the global lists)
+  // entries of this thread (-1: to be taken from the global lists; a call of one
+  // substep that reports the energy reads those themselves)
+  int n_ent = a.calc_epot && a.n_steps == 1 ? 0 : -1;
   bool fits = true;      // every thread's entries fit
   int rebuilds = 0;
   double epot = 0.0;

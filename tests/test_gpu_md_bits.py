@@ -27,13 +27,14 @@ CASES = {
 
 
 def _run(case, shape, calls):
-    arms, n_arm, frac, r_cut, r_verlet, pot, andersen = CASES[case]
+    """State after init_md and after every call, n substeps or (n, whether the energy is reported)."""
+    arms, n_arm, frac, r_cut, r_verlet, pot, andersen = case
     spec = system.ReplicaSpec(L=40, arms=arms, n_arm=n_arm, solvophobic_fraction=frac, shear=0.1, seed=71)
     st = system.make_star(arms, n_arm, frac, spec.mono_mass, spec.kT, np.random.default_rng(371), bond=0.97)
     desc = dict(W.replica_desc(spec, st), n_fluid=0, potential=pot, r_cut=r_cut, r_verlet=r_verlet)
     kw = dict(md_thermostat=capi.MDTHERMO_ANDERSEN, andersen_nu=1.0) if andersen else {}
     out = []
-    with capi.Context([desc], precision=capi.FP32, rng=capi.RNG_PHILOX, max_neighbors=512,
+    with capi.Context([desc], precision=capi.FP32, rng=capi.RNG_PHILOX, max_neighbors=1024,
                       step_update=W.N_SUB, strict_cells=0, **kw) as ctx:
         ctx.set_variants(0, 0, shape)
         ctx.set_monomers(0, st.pos, st.vel, np.zeros_like(st.pos), np.full(st.n, st.mass), st.amphi, st.anchor)
@@ -41,8 +42,9 @@ def _run(case, shape, calls):
         ctx.init_md()
         out.append(ctx.get_monomers(0))
         for n in calls:  # most calls begin with the lists of the one before
-            ctx.md_substeps(n)
-            out.append(ctx.get_monomers(0))
+            n, epot = n if isinstance(n, tuple) else (n, False)
+            ctx.md_substeps(n, calc_epot=epot)
+            out.append(ctx.get_monomers(0) + ((ctx.epot(0),) if epot else ()))
         if pot == LJ:  # (the reference's FENE reports bonds that a random start overstretches)
             ctx.raise_on_device_error()
         return out, ctx.verlet_rebuilds(0)
@@ -51,8 +53,24 @@ def _run(case, shape, calls):
 @pytest.mark.parametrize("case", list(CASES))
 def test_lists_in_shared_memory_give_the_same_bits(case):
     calls = (1, 3, 1, 10, 25)
-    (got, rebuilds), (want, expected) = (_run(case, shape, calls) for shape in (0, 1))
+    (got, rebuilds), (want, expected) = (_run(CASES[case], shape, calls) for shape in (0, 1))
     assert rebuilds == expected
     for g, w in zip(got, want):
         for a, b in zip(g, w):
             np.testing.assert_array_equal(a, b)
+
+
+# calls whose last substep reports the energy, from the lists of a call before (1), of
+# its own first substeps (3), after a rebuild; and lists that outgrow the shared memory
+@pytest.mark.parametrize("arms,n_arm,r_verlet", [(6, 20, 2.8), (10, 40, 2.8), (11, 93, 3.0), (12, 30, 9.0)])
+def test_substeps_that_report_the_energy_give_the_same_bits(arms, n_arm, r_verlet):
+    calls = ((1, True), (1, True), 5, (1, True), (3, True), 12, (1, True), 1)
+    case = (arms, n_arm, 0.5, 2.5, r_verlet, LJ, False)
+    (got, rebuilds), (want, expected) = (_run(case, shape, calls) for shape in (0, 1))
+    assert rebuilds == expected
+    for g, w in zip(got, want):
+        for a, b in zip(g, w):
+            if np.ndim(b):
+                np.testing.assert_array_equal(a, b)
+            else:  # the energy: terms of some 100 in all per bead, each of a few FP32 roundings
+                np.testing.assert_allclose(a, b, rtol=0, atol=100 * len(w[0]) * 4 * 2.0 ** -24)
