@@ -147,19 +147,21 @@ __global__ void __launch_bounds__(ANA_NT)
     part[6 * static_cast<size_t>(blockIdx.x) + threadIdx.x] = ri.solvent_mass * s_tot[threadIdx.x];
 }
 
-// Monomers of replica blockIdx.x, STRESS_LANES lanes per bead sharing its list;
-// block blockIdx.y of the replica's gridDim.y: kinetic part (6) and virial (6)
-// into part[12 (r gridDim.y + blockIdx.y)]. One block per replica left the
-// FP64 of all its pairs to one SM (120 us for 401 beads; 12 us split). Periodic boxes: their row lists and the minimum image at the
-// current delrx; other boxes: the transposed lists, plain differences.
+// One of a replica's blocks (blocks[blockIdx.x]: replica, its block, its number of
+// blocks), STRESS_LANES lanes per bead sharing its list: kinetic part (6) and
+// virial (6) into part[12 blockIdx.x]. One block per replica left the FP64 of all
+// its pairs to one SM (120 us for 401 beads; 12 us split). Periodic boxes: their
+// row lists and the minimum image at the current delrx; other boxes: the
+// transposed lists, plain differences.
 template <typename R>
 __global__ void __launch_bounds__(ANA_NT)
-    k_mono_stress(const RepInfo* reps, const RepDyn* dyn, const R* mpos, const R* mvel,
+    k_mono_stress(const int4* blocks, const RepInfo* reps, const RepDyn* dyn, const R* mpos, const R* mvel,
                   const int* nlist_t, const int* ncount, int n_mono_total, int* const* rows,
                   int max_nb, const int* bond_start, const int2* bonds, double* part) {
   __shared__ double s_red[12 * ANA_NT];
   __shared__ double s_tot[12];
-  const int r = blockIdx.x;
+  const int4 blk = blocks[blockIdx.x];
+  const int r = blk.x;
   const RepInfo& ri = reps[r];
   const int* row = rows[r];
   const bool periodic = (ri.flags & REP_PERIODIC_MD) != 0;
@@ -171,8 +173,8 @@ __global__ void __launch_bounds__(ANA_NT)
   double acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   double *kin = acc, *vir = acc + 6;
   const int sub = static_cast<int>(threadIdx.x) % STRESS_LANES;
-  for (int i = (blockIdx.y * ANA_NT + threadIdx.x) / STRESS_LANES; i < ri.n_mono;
-       i += gridDim.y * (ANA_NT / STRESS_LANES)) {
+  for (int i = (blk.y * ANA_NT + static_cast<int>(threadIdx.x)) / STRESS_LANES; i < ri.n_mono;
+       i += blk.z * (ANA_NT / STRESS_LANES)) {
     const size_t g = static_cast<size_t>(ri.mono_base) + i;
     const R4<R> x = ld4_rw(mpos, g), v = ld4_rw(mvel, g);
     if (sub == 0) {
@@ -221,16 +223,17 @@ __global__ void __launch_bounds__(ANA_NT)
   }
   block_sum_n<ANA_NT, 12>(acc, s_red, s_tot);
   if (threadIdx.x < 12)
-    part[12 * (static_cast<size_t>(r) * gridDim.y + blockIdx.y) + threadIdx.x] = s_tot[threadIdx.x];
+    part[12 * static_cast<size_t>(blockIdx.x) + threadIdx.x] = s_tot[threadIdx.x];
 }
 
-// A replica's partial sums into out[12 r]: a warp per component.
+// A replica's partial sums (spans[r]: first block, number of blocks) into
+// out[12 r]: a warp per component.
 template <typename R>  // R: the precision of the instantiating unit (one copy per unit)
-__global__ void k_stress_reduce(const double* part, int n_part, double* out) {
+__global__ void k_stress_reduce(const int2* spans, const double* part, double* out) {
   const int r = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int2 span = spans[r];
   double t = 0.0;
-  for (int q = lane; q < n_part; q += 32)
-    t += part[12 * (static_cast<size_t>(r) * n_part + q) + k];
+  for (int q = lane; q < span.y; q += 32) t += part[12 * (static_cast<size_t>(span.x) + q) + k];
   for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xFFFFFFFFu, t, o);
   if (lane == 0) out[12 * static_cast<size_t>(r) + k] = t;
 }

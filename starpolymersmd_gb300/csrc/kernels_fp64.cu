@@ -43,8 +43,12 @@ ProfilePlan profile_plan(int slots, size_t bins) {
   const bool copies = bins <= 65536 && static_cast<size_t>(slots) >= 50 * bins;
   return {copies ? std::max(1, std::min(128, blocks)) : 1, run};
 }
-int stress_parts(int n_mono) {
-  return std::max(1, std::min(1024, (n_mono * STRESS_LANES + ANA_NT - 1) / ANA_NT));
+// A block for every eight beads (one round of its 256 threads), or fewer where all
+// replicas' blocks would be more than eight per SM.
+int stress_blocks(int n_mono, long long total_mono) {
+  constexpr long long beads = ANA_NT / STRESS_LANES, most = 152 * 8;
+  const long long need = (n_mono + beads - 1) / beads, all = (total_mono + beads - 1) / beads;
+  return static_cast<int>(std::max(1ll, all <= most ? need : need * most / all));
 }
 int pmd_block_count(int n_beads) { return (n_beads + PMD_NT - 1) / PMD_NT; }
 }  // namespace smpc

@@ -226,13 +226,13 @@ template <>
 void launch_mono_stress<Real>(const RepInfo* reps, const RepDyn* dyn, int n_rep, const Real* mpos,
                               const Real* mvel, const int* nlist_t, const int* ncount,
                               int n_mono_total, int* const* rows, int max_nb,
-                              const int* bond_start, const int2* bonds, double* part,
-                              int n_part, double* out, cudaStream_t st) {
+                              const int* bond_start, const int2* bonds, const StressPlan& plan,
+                              cudaStream_t st) {
   if (n_rep == 0) return;
-  k_mono_stress<Real><<<dim3(n_rep, n_part), ANA_NT, 0, st>>>(reps, dyn, mpos, mvel, nlist_t,
-                                                              ncount, n_mono_total, rows, max_nb,
-                                                              bond_start, bonds, part);
-  k_stress_reduce<Real><<<n_rep, 12 * 32, 0, st>>>(part, n_part, out);
+  k_mono_stress<Real><<<plan.n_blocks, ANA_NT, 0, st>>>(plan.blocks, reps, dyn, mpos, mvel, nlist_t,
+                                                        ncount, n_mono_total, rows, max_nb,
+                                                        bond_start, bonds, plan.part);
+  k_stress_reduce<Real><<<n_rep, 12 * 32, 0, st>>>(plan.spans, plan.part, plan.out);
 }
 
 template <>

@@ -164,12 +164,21 @@ void launch_vacf_lags(const double* ring, int n_p, int entries, int first, doubl
 template <typename R>
 void launch_kinetic_tensor(const Tile* tiles, int n_tiles, const RepInfo* reps, const R* rec,
                            double* part, cudaStream_t st);
+// Blocks of launch_mono_stress: (replica, its block, its number of blocks, -),
+// and every replica's first block and number of blocks; part: 12 doubles per
+// block, out: 12 per replica.
+struct StressPlan {
+  int4* blocks = nullptr;
+  int2* spans = nullptr;
+  int n_blocks = 0;
+  double *part = nullptr, *out = nullptr;
+};
+int stress_blocks(int n_mono, long long total_mono);  // of a replica of n_mono beads of all
 template <typename R>
 void launch_mono_stress(const RepInfo* reps, const RepDyn* dyn, int n_rep, const R* mpos,
                         const R* mvel, const int* nlist_t, const int* ncount, int n_mono_total,
                         int* const* rows, int max_nb, const int* bond_start, const int2* bonds,
-                        double* part, int n_part, double* out, cudaStream_t st);
-int stress_parts(int n_mono);  // blocks (partial sums) per replica of launch_mono_stress
+                        const StressPlan& plan, cudaStream_t st);
 
 // Monomer state between the C ABI's x,y,z-interleaved doubles and the device
 // records (pos.w / vel.w keep mass and type): pos, vel, frc each 3M doubles, in

@@ -102,8 +102,7 @@ struct smpc_ctx {
   size_t ana_part_cap = 0;
   double* d_vacf_ring = nullptr;
   int** d_rows_by_rep = nullptr;  // each replica's periodic Verlet rows, or null
-  double* d_stress = nullptr;     // 12 per replica, then 12 per partial sum
-  int stress_parts = 1;           // partial sums per replica
+  smpc::StressPlan stress;        // the monomers' part of the pressure tensor
   int vacf_rep = -1, vacf_np = 0, vacf_entries = 0;
   uint64_t vacf_samples = 0, vacf_calcs = 0;
   std::vector<double> vacf_sum;
@@ -780,7 +779,9 @@ void free_all(smpc_ctx* ctx) {
   if (ctx->d_ana_part) cudaFree(ctx->d_ana_part);
   if (ctx->d_vacf_ring) cudaFree(ctx->d_vacf_ring);
   if (ctx->d_rows_by_rep) cudaFree(ctx->d_rows_by_rep);
-  if (ctx->d_stress) cudaFree(ctx->d_stress);
+  for (void* q : {static_cast<void*>(ctx->stress.blocks), static_cast<void*>(ctx->stress.spans),
+                  static_cast<void*>(ctx->stress.part), static_cast<void*>(ctx->stress.out)})
+    if (q) cudaFree(q);
   if (ctx->d_pamphi) cudaFree(ctx->d_pamphi);
   if (ctx->d_lowe) cudaFree(ctx->d_lowe);
   if (ctx->d_and_i) cudaFree(ctx->d_and_i);
@@ -995,9 +996,21 @@ int create_periodic_md(smpc_ctx* ctx) {
     CU(dalloc(&ctx->d_rows_by_rep, rows.size()));
     CU(cudaMemcpy(ctx->d_rows_by_rep, rows.data(), rows.size() * sizeof(int*),
                   cudaMemcpyHostToDevice));
-    for (const RepInfo& ri : ctx->reps)
-      ctx->stress_parts = std::max(ctx->stress_parts, smpc::stress_parts(ri.n_mono));
-    CU(dalloc(&ctx->d_stress, 12 * static_cast<size_t>(ctx->n_rep) * (1 + ctx->stress_parts)));
+    std::vector<int4> blocks;
+    std::vector<int2> spans;
+    for (int r = 0; r < ctx->n_rep; ++r) {
+      const int n = smpc::stress_blocks(ctx->reps[r].n_mono, ctx->total_mono);
+      spans.push_back(make_int2(static_cast<int>(blocks.size()), n));
+      for (int k = 0; k < n; ++k) blocks.push_back(make_int4(r, k, n, 0));
+    }
+    smpc::StressPlan& s = ctx->stress;
+    s.n_blocks = static_cast<int>(blocks.size());
+    CU(dalloc(&s.blocks, blocks.size()));
+    CU(dalloc(&s.spans, spans.size()));
+    CU(dalloc(&s.part, 12 * blocks.size()));
+    CU(dalloc(&s.out, 12 * spans.size()));
+    CU(cudaMemcpy(s.blocks, blocks.data(), blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(s.spans, spans.data(), spans.size() * sizeof(int2), cudaMemcpyHostToDevice));
   }
   if (!ctx->pmd.empty()) {
     CU(cudaMalloc(&ctx->d_pamphi, M));
@@ -2120,8 +2133,7 @@ int smpc_pressure_tensor_all(smpc_ctx* ctx, double* out) {
                                      static_cast<const double*>(ctx->d_mvel), ctx->d_nlist,
                                      ctx->d_ncount, static_cast<int>(ctx->total_mono),
                                      ctx->d_rows_by_rep, ctx->max_nb, ctx->d_bond_start,
-                                     ctx->d_bonds, ctx->d_stress + 12 * ctx->n_rep, ctx->stress_parts,
-                                     ctx->d_stress, ctx->st);
+                                     ctx->d_bonds, ctx->stress, ctx->st);
   } else {
     smpc::launch_kinetic_tensor<float>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps,
                                        static_cast<const float*>(ctx->d_rec[ctx->cur]),
@@ -2131,8 +2143,7 @@ int smpc_pressure_tensor_all(smpc_ctx* ctx, double* out) {
                                     static_cast<const float*>(ctx->d_mvel), ctx->d_nlist,
                                     ctx->d_ncount, static_cast<int>(ctx->total_mono),
                                     ctx->d_rows_by_rep, ctx->max_nb, ctx->d_bond_start,
-                                    ctx->d_bonds, ctx->d_stress + 12 * ctx->n_rep, ctx->stress_parts,
-                                     ctx->d_stress, ctx->st);
+                                    ctx->d_bonds, ctx->stress, ctx->st);
   }
   CU(cudaGetLastError());
   std::vector<double> part(6 * static_cast<size_t>(ctx->n_bin_tiles));
@@ -2140,7 +2151,7 @@ int smpc_pressure_tensor_all(smpc_ctx* ctx, double* out) {
   if (!part.empty())
     CU(cudaMemcpyAsync(part.data(), ctx->d_ana_part, part.size() * sizeof(double),
                        cudaMemcpyDeviceToHost, ctx->st));
-  CU(cudaMemcpyAsync(mono.data(), ctx->d_stress, mono.size() * sizeof(double),
+  CU(cudaMemcpyAsync(mono.data(), ctx->stress.out, mono.size() * sizeof(double),
                      cudaMemcpyDeviceToHost, ctx->st));
   CU(cudaStreamSynchronize(ctx->st));
   // the slot tiles' partial sums, tile by tile into their replicas
