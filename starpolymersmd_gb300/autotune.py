@@ -4,11 +4,14 @@ smpc_autotune (C ABI) times every launch-shape variant of the fast-path
 solvent-binning, collide and MD kernels (and of the periodic MD, in contexts
 with periodic boxes) on the context's own workload with CUDA events, keeps the
 fastest and restores the state its trial cycles advanced. This module caches
-the choice per GPU model and workload signature, so later runs of the same
-workload start tuned.
+the choice per GPU model, workload signature and kernel sources, so later runs
+of the same workload start tuned, and kernels that have changed are measured
+again.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 from typing import Optional
@@ -27,8 +30,19 @@ def gpu_name() -> str:
     return "unknown-gpu"
 
 
+@functools.lru_cache(maxsize=None)
+def kernels_id(folder: str = os.path.join(HERE, "csrc")) -> str:
+    """Digest of the kernel sources: what was fastest among other kernels need not be now."""
+    h = hashlib.sha256()
+    for name in sorted(n for n in os.listdir(folder) if n.endswith((".cu", ".cuh", ".h"))):
+        with open(os.path.join(folder, name), "rb") as f:
+            h.update(name.encode() + b"\0" + f.read() + b"\0")
+    return h.hexdigest()[:12]
+
+
 def signature(n_rep: int, particles: int, cells: int, monomers: int) -> str:
-    return f"{gpu_name()}|rep={n_rep}|particles={particles}|cells={cells}|monomers={monomers}"
+    return (f"{gpu_name()}|rep={n_rep}|particles={particles}|cells={cells}|monomers={monomers}"
+            f"|kernels={kernels_id()}")
 
 
 def _load(path: str) -> dict:
