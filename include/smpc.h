@@ -192,8 +192,9 @@ int smpc_cycles(smpc_ctx* ctx, int n);
 int smpc_cycles_profiled(smpc_ctx* ctx, int n, double* phase_ms, int n_phases, double* total_ms);
 /* Launch-shape variants of the FP32 fast-path kernels (solvent binning,
  * collide, MD substeps); index 0 is the default. The collide has one shape:
- * its indices 0 to 11 all name it. Changing them re-captures the cycle graph. FP64 contexts of few replicas run each replica's MD on a
- * cluster of SMs; md = 1 keeps one CTA per replica there instead. */
+ * its indices 0 to 11 all name it. Changing them re-captures the cycle graph.
+ * FP64 contexts of few replicas run each replica's MD on a cluster of SMs;
+ * md = 1 keeps one CTA per replica there instead. */
 int smpc_set_variants(smpc_ctx* ctx, int bin, int collide, int md);
 int smpc_get_variants(const smpc_ctx* ctx, int* bin, int* collide, int* md);
 /* Launch-shape variant of the periodic-MD kernels of FP32 contexts (lanes per
@@ -204,8 +205,9 @@ int smpc_get_pmd_variant(const smpc_ctx* ctx, int* pmd);
 /* Times every variant of each fast-path kernel (and, in contexts with periodic
  * boxes, of the periodic MD) over `cycles` cycles of the
  * context's own workload (CUDA events on the context stream), keeps the
- * fastest and writes a JSON report (variant -> ms per cycle, chosen). The
- * state is saved to host memory before the trials (as smpc_checkpoint_save)
+ * fastest and writes a JSON report (variant -> ms per cycle of the kernel, or
+ * of the whole captured cycle where that runs the kernel beside others: one
+ * periodic box; chosen). The state is saved to host memory before the trials (as smpc_checkpoint_save)
  * and restored after them, so the simulation does not advance. */
 int smpc_autotune(smpc_ctx* ctx, int cycles, char* report, int report_len);
 /* smpc_cycles bracketed by CUDA events on the context stream (ms). */
