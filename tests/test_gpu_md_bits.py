@@ -74,3 +74,31 @@ def test_substeps_that_report_the_energy_give_the_same_bits(arms, n_arm, r_verle
                 np.testing.assert_array_equal(a, b)
             else:  # the energy: terms of some 100 in all per bead, each of a few FP32 roundings
                 np.testing.assert_allclose(a, b, rtol=0, atol=100 * len(w[0]) * 4 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_forces_of_beads_far_from_the_first(sign):
+    # two straight arms side by side reach 80 list cells from bead 0; beads past 64 are
+    # listed in another order, so the sums of up to twenty terms below 60 round differently
+    n_arm = 110
+    k = np.arange(1, n_arm + 1)
+    arms = [np.stack([sign * 0.97 * k, np.full(n_arm, 1.05 * a), 0.03 * np.sin(1.0 * k)], axis=1) for a in range(2)]
+    pos = np.concatenate([[[0.0, 0.5, 0.0]], *arms])
+    n = len(pos)
+    src = np.concatenate([[0], np.arange(1, n_arm), [0], np.arange(n_arm + 1, n - 1)])
+    dst = np.concatenate([[1], np.arange(2, n_arm + 1), [n_arm + 1], np.arange(n_arm + 2, n)])
+    rep = dict(L=(300, 20, 20), n_fluid=0, n_mono=n, mol0_size=n, kT=1.0, shear=0.0, h=0.1, md_dt=0.01, seed=1,
+               potential=LJ, r_cut=1.13, r_verlet=1.3, **{"lambda": 1.0})
+    forces = []
+    for shape in (0, 1, 2):
+        with capi.Context([rep], precision=capi.FP32, rng=capi.RNG_PHILOX, step_update=1, strict_cells=0) as ctx:
+            ctx.set_variants(0, 0, shape)
+            ctx.set_monomers(0, pos, np.zeros_like(pos), np.zeros_like(pos), np.full(n, 5.0), np.zeros(n, np.int32),
+                             np.zeros(n, np.int32))
+            ctx.set_bonds(0, src, dst)
+            ctx.init_md()
+            ctx.raise_on_device_error()
+            forces.append(ctx.get_monomers(0)[2])
+    for f in (forces[0], forces[2]):
+        np.testing.assert_allclose(f, forces[1], rtol=0, atol=20 * 2.0 ** -24 * 60)
+    assert np.abs(forces[1][n_arm - 5:n_arm]).max() > 1.0
