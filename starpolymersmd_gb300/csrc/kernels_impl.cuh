@@ -116,9 +116,9 @@ void bin_f32(const Tile* tiles, int n_tiles, const RepInfo* reps, const FrameF* 
 
 template <>
 void launch_fluid_bin<Real>(const Tile* tiles, int n_tiles, const RepInfo* reps,
-                            const RepDyn* dyn, const FrameF* frames, const Real* rec, uint2* keys,
-                            uint32_t* count, ErrorState* err, int strict, int variant,
-                            int packed, Real* frame, const void* geo, cudaStream_t st) {
+                            const FrameF* frames, const Real* rec, uint2* keys, uint32_t* count,
+                            ErrorState* err, int strict, int variant, int packed, Real* frame,
+                            const void* geo, cudaStream_t st) {
   if (n_tiles == 0) return;
 #if SMPC_FAST_F32
   if (!strict && variant >= 0) {  // variant < 0: the generic kernel (what k_collide recomputes)
@@ -136,7 +136,7 @@ void launch_fluid_bin<Real>(const Tile* tiles, int n_tiles, const RepInfo* reps,
   (void)frames;
   (void)variant;
   k_fluid_bin<Real, SMPC_BIN_NT><<<n_tiles, SMPC_BIN_NT, 0, st>>>(
-      tiles, reps, dyn, rec, keys, count, err, strict, frame, static_cast<const Geo<Real>*>(geo));
+      tiles, reps, rec, keys, count, err, strict, frame, static_cast<const Geo<Real>*>(geo));
 }
 
 template <>

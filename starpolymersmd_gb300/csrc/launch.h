@@ -84,10 +84,9 @@ void launch_mono_prep(const RepInfo* reps, RepDyn* dyn, int n_rep, R* mpos, R* m
                       FrameF* frames, double rot_c, double rot_s, int chunks, int n_adv, double adv_scale,
                       int gen_shift, void* geo, int part, cudaStream_t st);
 template <typename R>
-void launch_fluid_bin(const Tile* tiles, int n_tiles, const RepInfo* reps, const RepDyn* dyn,
-                      const FrameF* frames, const R* rec, uint2* keys, uint32_t* count,
-                      ErrorState* err, int strict, int variant, int packed, R* frame,
-                      const void* geo, cudaStream_t st);
+void launch_fluid_bin(const Tile* tiles, int n_tiles, const RepInfo* reps, const FrameF* frames,
+                      const R* rec, uint2* keys, uint32_t* count, ErrorState* err, int strict,
+                      int variant, int packed, R* frame, const void* geo, cudaStream_t st);
 template <typename R>
 void launch_collide(const CollideArgs<R>& a, cudaStream_t st);
 template <typename R>

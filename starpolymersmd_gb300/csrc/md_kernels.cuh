@@ -1605,11 +1605,13 @@ template <typename R, int NT, int CS, int KMAX>
 __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel, R* mfrc, R* mver) {
   namespace cg = cooperative_groups;
   constexpr int CAP = MD_CLUSTER_CAP;
+  constexpr bool kF64 = sizeof(R) == 8;
   __shared__ unsigned char s_amphi[CAP];
-  __shared__ int s_head[MD_BUCKETS + 1];  // bucket starts in s_sorted
-  __shared__ int s_next[CAP];             // bucket of each bead
-  __shared__ int s_ckey[CAP];
-  __shared__ int s_sorted[CAP];
+  // the hash grid of FP32 list builds
+  __shared__ int s_head[kF64 ? 1 : MD_BUCKETS + 1];  // bucket starts in s_sorted
+  __shared__ int s_next[kF64 ? 1 : CAP];             // bucket of each bead
+  __shared__ int s_ckey[kF64 ? 1 : CAP];
+  __shared__ int s_sorted[kF64 ? 1 : CAP];
   __shared__ float s_coref[3];      // the core's position at the last rebuild (FP32)
   __shared__ int s_rebuild[2];      // by substep parity: a bead passed the Verlet limit
   __shared__ int s_farp[2];         // by substep parity: a coordinate reached MDC_FAR
@@ -1619,7 +1621,6 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
   static_assert((CAP + CS - 1) / CS <= NT, "a kick thread for every bead of the CTA");
   constexpr int NW = NT / 32;
   static_assert((NW & (NW - 1)) == 0, "a power of two of warps (candidate search)");
-  constexpr bool kF64 = sizeof(R) == 8;
   constexpr bool kBySum = kF64 && 3 * ((CAP + CS - 1) / CS) <= NT;  // a thread per force component
   using L = MdcLayout<R, CS>;
   __shared__ int s_wcnt[NW], s_woff[NW + 1];
@@ -1905,12 +1906,6 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
     }
     if (rebuild) {
       ++rebuilds;
-      // Membership is d^2 <= r_v^2 in the state's precision; FP64 states decide it
-      // in FP32 outside a band of 2^-7 around r_v^2 (FP32 rounding of
-      // coordinates below MDC_FAR moves d^2 by far less) and in FP64 inside it.
-      const bool fast = kF64 && !far_now;
-      const float rv2_lo = static_cast<float>(rv2) * (1.0f - 0.0078125f);
-      const float rv2_hi = static_cast<float>(rv2) * (1.0f + 0.0078125f);
       // list starts of the CTA's beads, from their lengths in s_cstart
       auto list_starts = [&]() {
         if (threadIdx.x < 32) {
@@ -1928,7 +1923,13 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
           }
         }
       };
-      if (kF64) {
+      // Membership is d^2 <= r_v^2 in the state's precision; FP64 states decide it
+      // in FP32 outside a band of 2^-7 around r_v^2 (FP32 rounding of
+      // coordinates below MDC_FAR moves d^2 by far less) and in FP64 inside it.
+      if constexpr (kF64) {
+        const bool fast = !far_now;
+        const float rv2_lo = static_cast<float>(rv2) * (1.0f - 0.0078125f);
+        const float rv2_hi = static_cast<float>(rv2) * (1.0f + 0.0078125f);
         // A CTA owns n / CS beads: testing each against all n, a warp 128 at a
         // time, takes 15,000 cycles for 25 of 401 with everything around it;
         // sorting all n into hash cells in every CTA and walking 27 of them
@@ -2007,12 +2008,10 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
       // lanes), count their members, then write them at the offsets the
       // counts give, so a list holds lane 0's cells, then lane 1's, and so on.
       int ccx = 0, ccy = 0, ccz = 0;
-      float xf0 = 0.f, xf1 = 0.f, xf2 = 0.f;
       if (mine) {
         ccx = static_cast<int>(floor(x[0] * inv_rv));
         ccy = static_cast<int>(floor(x[1] * inv_rv));
         ccz = static_cast<int>(floor(x[2] * inv_rv));
-        xf0 = pxf[i]; xf1 = pyf[i]; xf2 = pzf[i];
       }
       // members of this lane's cells: counted (pos < 0) or written from pos
       // emit(j) for every member of this lane's cells, in order; members
@@ -2025,32 +2024,16 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
           const int kend = s_head[bk + 1];
           for (int kk = s_head[bk]; kk < kend; kk += 4) {
             int jj[4], kc[4];
-            float e0[4], e1[4], e2[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) jj[u] = kk + u < kend ? s_sorted[kk + u] : -1;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const int j = jj[u] < 0 ? 0 : jj[u];
-              kc[u] = s_ckey[j];
-              e0[u] = pxf[j] - xf0;
-              e1[u] = pyf[j] - xf1;
-              e2[u] = pzf[j] - xf2;
-            }
+            for (int u = 0; u < 4; ++u) kc[u] = s_ckey[jj[u] < 0 ? 0 : jj[u]];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               const int j = jj[u];
               if (j < 0 || j == i || kc[u] != want) continue;
-              bool in;
-              const float r2f = fmaf(e0[u], e0[u], fmaf(e1[u], e1[u], e2[u] * e2[u]));
-              if (fast && r2f < rv2_lo) {
-                in = true;
-              } else if (fast && r2f > rv2_hi) {
-                in = false;
-              } else {
-                const R d0 = sx[j] - x[0], d1 = sy[j] - x[1], d2 = sz[j] - x[2];
-                in = (d0 * d0 + d1 * d1) + d2 * d2 <= rv2;
-              }
-              if (in) emit(j);
+              const R d0 = sx[j] - x[0], d1 = sy[j] - x[1], d2 = sz[j] - x[2];
+              if ((d0 * d0 + d1 * d1) + d2 * d2 <= rv2) emit(j);
             }
           }
         }

@@ -750,7 +750,7 @@ __device__ __forceinline__ uint32_t word_key(float w) { return __float_as_uint(w
 // narrow FP64 pipe; the arithmetic is the same).
 template <typename R, int NT>
 __global__ void __launch_bounds__(NT) k_fluid_bin(const Tile* tiles, const RepInfo* reps,
-                                                  const RepDyn* dyn, const R* __restrict__ st,
+                                                  const R* __restrict__ st,
                                                   uint2* __restrict__ keys, uint32_t* count,
                                                   ErrorState* err, int strict, R* frame,
                                                   const Geo<R>* geo) {

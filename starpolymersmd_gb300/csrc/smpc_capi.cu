@@ -229,10 +229,9 @@ void launch_prep(smpc_ctx* ctx, int n_adv, double adv, int gen_shift, int part, 
 
 template <typename R>
 void launch_solvent_binning(smpc_ctx* ctx, int cur, cudaStream_t st) {
-  smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_dyn,
-                            ctx->d_frames, static_cast<const R*>(ctx->d_rec[cur]), ctx->d_keys,
-                            ctx->d_count, ctx->d_err, ctx->opt.strict_cells,
-                            ctx->opt.angular_momentum ? -1 : ctx->var_bin,
+  smpc::launch_fluid_bin<R>(ctx->d_bin_tiles, ctx->n_bin_tiles, ctx->d_reps, ctx->d_frames,
+                            static_cast<const R*>(ctx->d_rec[cur]), ctx->d_keys, ctx->d_count,
+                            ctx->d_err, ctx->opt.strict_cells, ctx->opt.angular_momentum ? -1 : ctx->var_bin,
                             ctx->packed_keys ? 1 : 0, static_cast<R*>(ctx->d_frame), ctx->d_geo, st);
   ctx->frame_ok = ctx->d_frame != nullptr;
 }
