@@ -1,6 +1,8 @@
 // FP64 reference-parity instantiation. Built with -fmad=false so every
-// multiply and add rounds separately, in the reference's order; only the
-// collision itself (cell sums, rotation) writes out fused operations.
+// multiply and add rounds separately, in the reference's order. Fused operations
+// are written out in the collision itself (cell sums, rotation with the
+// thermostat's factor), the gamma variate and the kinetic stress; the cluster MD
+// adds a bead's even and odd force terms apart.
 #define SMPC_REAL double
 #define SMPC_FAST_F32 0
 #define SMPC_COLLIDE_NT 128

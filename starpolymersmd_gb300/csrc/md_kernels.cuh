@@ -872,7 +872,8 @@ __device__ __noinline__ void md_bead_forces_lists(const MdArgs& a, int b, int i,
 // The FP32 substeps of one replica per CTA with the lists in shared memory
 // (no Lowe-Andersen; at most NT beads). Results are those of k_md_substeps
 // with one bead per thread and up to KMAX lanes per bead, to the last bit:
-// the Verlet lists, their order and the order of every sum are the same.
+// the Verlet lists, their order and the order of every sum are the same (while
+// all beads lie within 64 list cells of bead 0; further out the order differs).
 //
 //  * Lists: each thread keeps its share of its bead's list in shared memory,
 //    without the pairs that cannot come into range before the next rebuild:

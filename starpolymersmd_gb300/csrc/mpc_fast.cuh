@@ -437,7 +437,7 @@ __device__ __forceinline__ float row_apply(const float4& r, float d0, float d1, 
 //           folded into the cell's rotation;
 //  apply  : v' = cmv + sR (v - cmv), back to the primary box, written in cell
 //           order as 32-byte records.
-// What bounds it: instruction issue (59 % of the slots; 10.7 warp
+// What bounds it: instruction issue (60 % of the slots; 11.1 warp
 // instructions per particle), then the latency of the phases. Small CTAs keep
 // more of them in different phases and their barriers cheap: 16 CTAs of 64
 // threads and 32 cells fit one SM and ran at 935 us for 65.8 M particles,

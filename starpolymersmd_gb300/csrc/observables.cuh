@@ -201,14 +201,14 @@ __global__ void __launch_bounds__(NT) k_mol_observables(const int2* mols, const 
   o[14] = dn;
 }
 
-// One thread per replica: its molecules' values in molecule order. out[16 r
+// One warp per replica: means over its molecules. out[16 r
 // + ...]: mean R_g, mean G (row-major, 9), mean rotation frequency (3),
 // kinetic energy, temperature 2 E / (3 (N - 1)), molecules.
 template <typename R>  // R: the precision of the instantiating unit (one copy per unit)
 __global__ void k_obs_reduce(const int2* rep_mols, const double* mol_out, int n_rep, double* out) {
   // one warp per replica: lane l sums molecules l, l + 32, ... in order, then
-  // a fixed xor butterfly joins the lanes (every lane ends with the same bits;
-  // a replica of one molecule gets its values unchanged)
+  // a fixed xor butterfly joins the lanes; lane 0 writes (a replica of one
+  // molecule gets its values unchanged)
   constexpr unsigned FULL = 0xFFFFFFFFu;
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
