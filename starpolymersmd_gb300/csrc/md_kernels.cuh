@@ -1774,7 +1774,11 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
   // the half-kick increment f / m dt / 2 (Thermostat_None.cpp:22,34), taken
   // once per force evaluation: the second half-kick of a substep and the
   // first of the next use the same force
-  R fk[3] = {R(0), R(0), R(0)};
+  R fk[3] = {R(0), R(0), R(0)}, c_andersen = R(0), rm = R(1);
+  auto increment = [&]() {
+    for (int d = 0; d < 3; ++d)
+      fk[d] = a.andersen ? f[d] * c_andersen : (kF64 ? div_exact(f[d], m, rm) : f[d] / m) * dth;
+  };
   if (kicker) {
     const R4<R> p = ld4_rw(mpos, b + ik), vv = ld4_rw(mvel, b + ik), ff = ld4_rw(mfrc, b + ik),
                 pv = ld4_rw(mver, b + ik);
@@ -1782,14 +1786,15 @@ __global__ void __launch_bounds__(NT, 1) k_md_cluster(MdArgs a, R* mpos, R* mvel
     v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
     f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
     xv[0] = pv.x; xv[1] = pv.y; xv[2] = pv.z;
+    // dth / m or 1 / m once (the quotients have the division's bits), by the few
+    // warps of the kick threads: in all of them the divisions were a microsecond
+    // of the narrow pipe
+    if (a.andersen)
+      c_andersen = dth / m;
+    else if (kF64)
+      rm = R(1) / m;
+    increment();
   }
-  // (dth / m and 1 / m once; the quotients have the division's bits)
-  const R c_andersen = dth / m, rm = kF64 ? R(1) / m : R(1);
-  auto increment = [&]() {
-    for (int d = 0; d < 3; ++d)
-      fk[d] = a.andersen ? f[d] * c_andersen : (kF64 ? div_exact(f[d], m, rm) : f[d] / m) * dth;
-  };
-  increment();
   // FP64 Andersen draws (not staged ones) depend on the counters only: the
   // upper half of the block makes them beside the lower half's force sums,
   // two threads per bead, instead of each kick thread after its force, where
