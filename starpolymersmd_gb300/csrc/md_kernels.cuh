@@ -977,7 +977,9 @@ static __device__ __noinline__ void md_bead_forces_global(const MdArgs& a, int b
   const int cnt = a.ncount[b + i];
   const int* nl = a.nlist + b + i;
   const size_t stride = static_cast<size_t>(a.n_mono_total);
-  constexpr int PF = 4;  // list loads in flight (8 cost the caller registers)
+  // list loads in flight: a substep of 709 beads that reports the energy took 46 us
+  // with one, 39 with four (eight cost the caller registers)
+  constexpr int PF = 4;
   double ep = 0.0;
 #pragma unroll 1
   for (int q0 = sub; q0 < cnt; q0 += PF << lk) {
@@ -1407,7 +1409,8 @@ __global__ void __launch_bounds__(NT, NT == 512 && KMAX > 1 ? 2 : 1)
     }
   }
   // entries of this thread (-1: to be taken from the global lists; a call of one
-  // substep that reports the energy reads those themselves)
+  // substep that reports the energy reads those themselves: 709 beads 39 us
+  // after a pass that takes them, 34 without)
   int n_ent = a.calc_epot && a.n_steps == 1 ? 0 : -1;
   bool fits = true;      // every thread's entries fit
   int rebuilds = 0;

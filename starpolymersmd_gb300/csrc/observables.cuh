@@ -486,7 +486,7 @@ __device__ __forceinline__ void prof_add(ProfAcc& even, ProfAcc& odd, long long 
 // collision, so a run meets a few bins only, two neighbouring ones per axis at
 // a time; their sums stay in registers (one pair for even bins, one for odd)
 // and go out when the bin changes. One atomic per particle and sum onto the
-// few hundred addresses took 1015 us for 1.25 M particles; this takes 124 with
+// few hundred addresses took 1015 us for 1.25 M particles; this takes 115 with
 // the slots in id order, where every particle changes the bin. Wraps and bins
 // are decided without divisions.
 template <typename R>
